@@ -44,6 +44,56 @@ enum OpenSection : int {
   OPEN_ALL = 255
 };
 
+// Coefficients of the strip kernel's node quantities and face fluxes
+// (dim2d_strip.cu), from the physical constants and the grid step: computed
+// on the host once per launch so that the kernel reads them as constants.
+constexpr int STRIP_COLS = 30;  // interior columns of one strip
+template <typename T>
+struct FaceCoef {    // n = face normal, t = tangential
+  T s;               // sqrt(1/We) / dn
+  T dn, dt;          // 1/dn, 1/(4 dt)
+  T a1, a2;          // (2 + mu)/(Re dn), mu/(4 Re dt)
+  T b1, b2;          // 1/(4 Re dt), 1/(Re dn)
+  T th;              // 2/(Re Pr dn)
+};
+template <typename T>
+struct StripCoef {
+  FaceCoef<T> x, y;
+  T s;               // sqrt(1/We)
+  T c15cv;           // 1.5/cv_r
+  T gx, gy;          // sqrt(1/We)/(4 dx), .../(4 dy)
+  T lx, ly;          // 1/(2 We dx^2), 1/(2 We dy^2)
+};
+inline FaceCoef<double> face_coef(const DimConst& k, double s, double rdn, double rdt) {
+  return FaceCoef<double>{s * rdn,
+                          rdn,
+                          0.25 * rdt,
+                          k.ire * k.two_mu * rdn,
+                          0.25 * k.ire * k.viscous_r * rdt,
+                          0.25 * k.ire * rdt,
+                          k.ire * rdn,
+                          2.0 * k.irepr * rdn};
+}
+inline StripCoef<double> strip_coef_of(const DimConst& k, double rdx, double rdy) {
+  const double s = sqrt(k.iwe);
+  return StripCoef<double>{face_coef(k, s, rdx, rdy),
+                           face_coef(k, s, rdy, rdx),
+                           s,
+                           k.c15cv,
+                           0.25 * s * rdx,
+                           0.25 * s * rdy,
+                           0.5 * k.iwe * rdx * rdx,
+                           0.5 * k.iwe * rdy * rdy};
+}
+__host__ __device__ inline FaceCoef<float> face_coef_f32(const FaceCoef<double>& c) {
+  return FaceCoef<float>{(float)c.s,  (float)c.dn, (float)c.dt, (float)c.a1,
+                         (float)c.a2, (float)c.b1, (float)c.b2, (float)c.th};
+}
+__host__ __device__ inline StripCoef<float> strip_coef_f32(const StripCoef<double>& c) {
+  return StripCoef<float>{face_coef_f32(c.x), face_coef_f32(c.y), (float)c.s,  (float)c.c15cv,
+                          (float)c.gx,        (float)c.gy,        (float)c.lx, (float)c.ly};
+}
+
 struct StageArgs {
   const double* __restrict__ uin;  // state the stencil reads
   const double* __restrict__ u0;   // u^n (stages 2 and 3)
@@ -73,6 +123,8 @@ struct StageArgs {
   int box_x0, box_x1, box_y0, box_y1;
   WallConst wall;
   DimConst k;
+  StripCoef<double> c;                 // strip kernels
+  StripCoef<float> cf;                 // ... and their FP32 face pass (mixed)
 };
 
 // sides of StageArgs::node_sides
@@ -183,6 +235,7 @@ struct BatchDomain {
   int open;                // OPEN_* mask of the time-integrated ghost sections
   int node_sides;          // as StageArgs::node_sides
   int ghost0, strip0, sx;  // first ghost CTA, first strip CTA, strips per row
+  StripCoef<double> c;
 };
 
 struct BatchStageArgs {
@@ -253,6 +306,7 @@ struct PDomain {
   int band0;                                         // first of its band counters
   int nn;                                            // node items per stage (0: no pass)
   unsigned int* status;                              // wall root status word
+  StripCoef<double> c;
 };
 
 struct PItem {

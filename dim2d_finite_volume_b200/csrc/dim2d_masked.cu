@@ -113,6 +113,7 @@ int dim2d_time_dev_masked(const dim2d_params* p, int nx, int ny, const double* n
   a.rdx = 1.0 / dx;
   a.rdy = 1.0 / dy;
   a.k = make_const(*p);
+  a.c = strip_coef_of(a.k, a.rdx, a.rdy);
   const cudaError_t e = launch_time_dev_masked(a, static_cast<cudaStream_t>(stream));
   if (e != cudaSuccess) return cuda_error(e, "time_dev_masked");
   return DIM2D_OK;

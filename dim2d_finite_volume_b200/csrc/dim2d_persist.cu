@@ -169,7 +169,8 @@ int persist_build(PersistPlan& pl, const std::vector<dim2d_handle*>& hs,
     d.open_e = h->open_e;
     d.open_n = h->open_n;
     d.status = h->status;
-    d.sx = (h->f.nx - 2 * BC + 29) / 30;  // 30 interior columns per strip
+    d.c = strip_coef_of(h->k, h->rdx, h->rdy);
+    d.sx = (h->f.nx - 2 * BC + STRIP_COLS - 1) / STRIP_COLS;
     d.nb = band_count(h->f.ny - 2 * BC, rows);
     d.band0 = (int)sg.size();
     d.nn = (h->periodic || h->open_all) ? 0 : (node_bc_count(node_args_of(h)) + 31) / 32;

@@ -41,6 +41,8 @@ StageArgs make_stage_args(const dim2d_handle* h, const double* uin, double* uout
   a.node_sides = st >= 2 ? h->node_sides : 0;
   a.wall = h->wall;
   a.k = h->k;
+  a.c = strip_coef_of(h->k, h->rdx, h->rdy);
+  a.cf = strip_coef_f32(a.c);
   return a;
 }
 

@@ -1,30 +1,40 @@
 // dim2d_strip.cu -- fused RK3 stage, warp-streaming variant for sm_100a.
 //
-// Same physics as k_interior (dim2d_interior.cu) -- node quantities, face
-// fluxes, divergence, body force, stage update -- organised so that no
-// CTA-wide barrier is needed and every face and node quantity is computed
-// once:
-//   * a warp owns a strip of 30 interior columns (lane = column) and H rows
-//     and marches up the strip one row per iteration;
-//   * per-warp shared-memory rings hold 3 rows of the input state (rows
-//     y..y+2, 34 columns), 3 rows of velocities (y-1..y+1) and 2 rows of
-//     the other node quantities (y, y+1) for 32 columns -- one per lane, so
-//     the node pass is a single warp pass;
-//   * node quantities: u, v, P, Tcl, 1/(3-rho), Tcap, and the node
-//     Laplacian and centred gradient of rho.  The face Laplacian and
-//     tangential density derivative of the reference's Mattsson stencils
-//     are the averages of the two nodes' values (the same sums, regrouped);
-//   * iteration y: issue the global loads of row y+3 (prefetch into
-//     registers), compute the node quantities of row y+1, then the x-face
-//     between columns x-1 and x of row y and the y-face between rows y and
-//     y+1 of column x; the right x-face of the cell comes from lane+1 by a
-//     shuffle, the bottom y-face is the top face of the previous iteration
-//     (kept in registers); update cell (x, y); store the prefetched row
-//     into the ring slot of row y.
-// Lane 30 evaluates only the x-face its left neighbour needs; lane 31's
-// face work repeats lane 30's / 29's (clamped column, result unused).
-// Warps are independent (__syncwarp only), so the latency of one warp's
-// loads is hidden by the arithmetic of the others.
+// Node quantities, face fluxes, divergence, body force and stage update of
+// one RK stage (or the time derivative) in one pass over the state:
+//   * a warp owns a strip of 30 interior columns and H rows and marches up
+//     the strip one row per iteration; lane l holds column c0-1+l, so lanes
+//     1..30 own the cells and lanes 0 and 31 their neighbours;
+//   * what a cell needs of its own column stays in the lane's registers:
+//     the state of row y, the node quantities of rows y and y+1, the bottom
+//     face's flux.  What it needs of the columns beside it comes by warp
+//     shuffle; state rows and u^n rows travel ahead of the warp into a
+//     shared-memory ring (cp.async);
+//   * node quantities (NodeQ) are chosen so that a face flux is made of their
+//     sums and differences: products such as my v + P, rho u v and
+//     (E + P) v are taken once per node instead of twice per face, and
+//     Tcl - Tcap/We is one quantity, since both enter the energy flux by
+//     their normal derivative with the factor 1/(Re Pr).  sqrt(1/We) is
+//     folded into the density gradients, 1/We into the Laplacian.  Face
+//     Laplacian and tangential derivatives are the sums of the two nodes'
+//     halves (the reference's Mattsson stencils, regrouped);
+//   * iteration y: copies of rows y+4 (state) and y+2 (u^n) are issued;
+//     velocities of row y+1; x-face between columns x-1 and x of row y; the
+//     other node quantities of row y+1; y-face between rows y and y+1; the
+//     right x-face comes from lane+1, the bottom y-face is the top one of the
+//     iteration before; update of cell (x, y).  Two rows per pass of the
+//     loop, so that the values handed from row to row need no moves.
+//
+// Bound: instruction issue and FP64 latency at 4 warps per scheduler.  The
+// form before this one kept node quantities in shared memory too and moved
+// 165 128-byte wavefronts per warp and row through that pipe, against 121
+// cycles of FP64 work; now a row costs 34 shuffles, 36 wavefronts of row data
+// and 165 FP64 instructions instead of 242.  Measured per RK3 step (best
+// shape): 1024^2 periodic 99.7 -> 74.5 us, 2048^2 open 321.7 -> 244.3 us,
+// 2048^2 wall in mixed precision 324.8 -> 221.2 us.  Tried beside it: all
+// rows prefetched into registers instead of the ring (periodic 85.7, more
+// registers and 420 instead of 400 instructions per row), 20 warps per SM at
+// 96 registers (92; spills), three or four rows per pass (as fast, larger).
 //
 // On a field with open sections the launch also integrates their ghost
 // cells (open_ghost_cell, one thread each): they take the first CTAs of the
@@ -40,35 +50,40 @@ namespace dim2d {
 
 namespace {
 
-constexpr int SW = 30;  // cells per strip
-constexpr int RC = 34;  // state columns in the ring: c0-2 .. c0+31
-constexpr int PC = 34;  // node-quantity columns: c0-1 .. c0+32 (the last two are
-                        // padding read only by lane 31, whose faces are unused)
-constexpr int NS = 4;   // state rows (y .. y+2, and the row y+3 landing)
-constexpr int NUV = 3;  // velocity rows (y-1 .. y+1)
-constexpr int NQ = 2;   // rows of the other node quantities (y, y+1)
-// node quantities besides u, v; GXH/GYH = half the centred density
-// gradient, LAPH = half the density Laplacian
-enum NodeQ : int { Q_P = 0, Q_TCL, Q_CP, Q_TCAP, Q_LAPH, Q_GXH, Q_GYH, NQV };
-constexpr int ST_ROW = 4 * RC;    // doubles per state row (4 variables)
-constexpr int UV_ROW = 2 * PC;    // doubles per velocity row
-constexpr int Q_ROW = NQV * PC;   // doubles per node-quantity row
-constexpr int UN_ROW = 4 * 32;    // u^n of one row of the strip's cells (4 variables)
-constexpr int WARP_DOUBLES = NS * ST_ROW + NUV * UV_ROW + NQ * Q_ROW + 2 * UN_ROW;
+constexpr int SW = STRIP_COLS;  // cells per strip
+constexpr int WARPS = 16;       // resident warps per SM (one warp per CTA, <= 128 registers)
 
-extern __shared__ __align__(16) double g_ring[];
+// A stage launched as a programmatic dependent of the node pass before it
+// (StageArgs::node_sides != 0) starts while that pass runs: a warp whose
+// rows or columns reach a side the pass writes waits for the pass (and its
+// memory) before its first read; the other warps read only cells the
+// previous stage wrote, complete before the pass began.
+__device__ __forceinline__ void wait_for_node_pass() {
+  asm volatile("griddepcontrol.wait;\n" ::: "memory");
+}
+// 1 if the warp's reads -- columns c0-2 .. c0+31, rows y0-2 .. y1+1,
+// clamped to the field -- reach a ghost cell of the sides in `sides`
+__device__ __forceinline__ bool reads_node_ghosts(int sides, const Field& f, int c0, int y0,
+                                                  int y1) {
+  return ((sides & NODE_W) && c0 - 2 < BC) || ((sides & NODE_E) && c0 + 31 >= f.nx - BC) ||
+         ((sides & NODE_S) && y0 - 2 < BC) || ((sides & NODE_N) && y1 + 1 >= f.ny - BC);
+}
 
-// Ring rows are addressed by offsets into g_ring that already include the
-// warp's base and the lane's column; the offsets rotate as the warp moves
-// up, so every access below is a register plus a compile-time constant.
-#define ST(o, v, dc) g_ring[(o) + (v) * RC + (dc)]
-#define UV(o, c, dc) g_ring[(o) + (c) * PC + (dc)]
-#define NQ_(o, c, dc) g_ring[(o) + (c) * PC + (dc)]
+template <typename T>
+__device__ __forceinline__ T from_left(T v) {
+  return __shfl_up_sync(0xffffffffu, v, 1);
+}
+template <typename T>
+__device__ __forceinline__ T from_right(T v) {
+  return __shfl_down_sync(0xffffffffu, v, 1);
+}
 
-// Asynchronous global -> shared copies (cp.async): the next state row and
-// the next row's u^n land in the ring while the warp computes, without
-// passing through registers.  Completion is per thread (commit / wait
-// groups); a __syncwarp after the wait makes the whole row visible.
+// Asynchronous global -> shared copies (cp.async) through L2: the state rows
+// and u^n rows ahead of the warp land in its shared-memory ring while it
+// computes, without passing through registers.  (The L2 path is coherent:
+// the persistent kernel rereads buffers that other SMs rewrite within its
+// launch.)  Completion is per thread (commit / wait groups); a __syncwarp
+// after the wait makes the whole row visible.
 __device__ __forceinline__ void cp_async16(double* smem, const double* gmem) {
   const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(sa), "l"(gmem) : "memory");
@@ -82,531 +97,477 @@ __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
 }
 
-// A stage launched as a programmatic dependent of the node pass before it
-// (StageArgs::node_sides != 0) starts while that pass runs: a warp whose
-// rows or columns reach a side the pass writes waits for the pass (and its
-// memory) before its first read; the other warps read only cells the
-// previous stage wrote, complete before the pass began.
-__device__ __forceinline__ void wait_for_node_pass() {
-  asm volatile("griddepcontrol.wait;\n" ::: "memory");
-}
-// 1 if the warp's reads -- columns c0-2 .. c0+31, rows y0-2 .. y1+2 (the
-// last one a prefetch past the strip), clamped to the field -- reach a
-// ghost cell of the sides in `sides`
-__device__ __forceinline__ bool reads_node_ghosts(int sides, const Field& f, int c0, int y0,
-                                                  int y1) {
-  return ((sides & NODE_W) && c0 - 2 < BC) || ((sides & NODE_E) && c0 + 31 >= f.nx - BC) ||
-         ((sides & NODE_S) && y0 - 2 < BC) || ((sides & NODE_N) && y1 + 2 >= f.ny - BC);
-}
+// The warp's ring: NS state rows (columns c0-2 .. c0+31 of 4 planes) and NU
+// rows of u^n (columns c0-2 .. c0+29, same row length).
+constexpr int RC = 34, NS = 5, NU = 3;
+constexpr int ST_ROW = 4 * RC, UN_ROW = ST_ROW;
+constexpr int WARP_DOUBLES = NS * ST_ROW + NU * UN_ROW;
+extern __shared__ __align__(16) double g_ring[];
 
-// state row `row` into the ring row at offset o (which includes the lane),
-// asynchronously: lane p < 17 copies the 16-byte pairs of columns
-// c0-2+2p, c0-1+2p of the 4 planes.  Addresses are clamped to the field's
-// rows and to its pitch, so no copy leaves the allocation; the clamped
-// values land in ring columns that only unused lanes read.  Needs an even
-// pitch and 16-byte aligned planes (strip_layout_ok).
-__device__ __forceinline__ void async_row(const StageArgs& a, int c0, int row, int lane, int o) {
-  if (lane < 17) {
-    const int r = min(row, a.f.ny - 1);
-    const int xp = min(c0 - 2 + 2 * lane, a.f.pitch - 2);
-    const double* src = a.uin + (size_t)r * a.f.pitch + xp;
-    double* dst = g_ring + (o - lane) + 2 * lane;
-#pragma unroll
-    for (int q = 0; q < 4; q++) cp_async16(dst + q * RC, src + q * a.f.plane);
+// The lane's part in copying a row: 16-byte pairs of columns c0-2 .. c0+29
+// of two planes at once (lanes 0-15 one plane, 16-31 the next) and, by lanes
+// 0..3, the pair of columns c0+30, c0+31 of one plane each.  Columns are
+// clamped to the pitch, so no copy leaves the allocation; clamped values land
+// in columns that only unused lanes read.  Needs an even pitch and 16-byte
+// aligned planes (strip_layout_ok).
+struct RowCopy {
+  const double* src;  // the lane's first pair in the next row to copy
+  size_t edge;        // from there to its pair of columns c0+30, c0+31
+  int dst, edge_dst;  // their places in a ring row
+  __device__ __forceinline__ RowCopy(const double* u, const Field& f, int c0, int row, int lane) {
+    const int half = lane >> 4, pair = 2 * (lane & 15);
+    const int col = min(c0 - 2 + pair, f.pitch - 2);
+    src = u + (size_t)row * f.pitch + half * f.plane + col;
+    edge = (size_t)lane * f.plane + (min(c0 + 30, f.pitch - 2) - col);
+    dst = half * RC + pair;
+    edge_dst = lane * RC + 32;
   }
-}
-
-// u^n of row y, columns c0 .. c0+31, into the u^n ring row at offset un
-// (which includes the lane): lane p < 16 copies the 16-byte pair of columns
-// c0+2p, c0+2p+1 of the 4 planes through L2 (cp.async.cg; the persistent
-// kernel rereads u^n buffers that other SMs rewrite within its launch, and
-// the L2 path is coherent).  Addresses clamped to the pitch like async_row.
-__device__ __forceinline__ void async_un(const StageArgs& a, int c0, int y, int un, int lane) {
-  if (lane < 16) {
-    const int xp = min(c0 + 2 * lane, a.f.pitch - 2);
-    const double* src = a.u0 + (size_t)y * a.f.pitch + xp;
-    double* dst = g_ring + (un - lane) + 2 * lane;
-#pragma unroll
-    for (int v = 0; v < 4; v++) cp_async16(dst + v * 32, src + v * a.f.plane);
+  // the next state row into the ring row at `to`
+  __device__ __forceinline__ void state(const Field& f, double* to, int lane) const {
+    cp_async16(to + dst, src);
+    cp_async16(to + dst + 2 * RC, src + 2 * f.plane);
+    if (lane < 4) cp_async16(to + edge_dst, src + edge);
   }
-}
-
-// node quantities of column c0-1+lane of one row: sm/s0/sp = state rows
-// below / at / above, ou/oq = output rows.  Primitives as node_prim()
-// (dim2d_prim_module.f:242-289, 425-453, 515-544, 1056-1071) with 1/rho
-// and 1/(3-rho) from one division; Tcap = 0.5/rho |grad rho|^2 with
-// centred gradients (:582-613).
-__device__ __forceinline__ void node_row(int sm, int s0, int sp, int ou, int oq, double qrdx,
-                                         double qrdy, double hrdx2, double hrdy2,
-                                         const DimConst& k) {
-  const double r = ST(s0, 0, 1);
-  const double rw = ST(s0, 0, 0), re = ST(s0, 0, 2);
-  const double rs = ST(sm, 0, 1), rn = ST(sp, 0, 1);
-  const double tm = 3.0 - r;
-  const double inv = 1.0 / (r * tm);
-  const double ir = tm * inv;
-  const double cp = r * inv;
-  const double u = ST(s0, 1, 1) * ir, v = ST(s0, 2, 1) * ir;
-  const double w = ST(s0, 3, 1) - 0.5 * r * (u * u + v * v) + 3.0 * (r * r);
-  const double gxh = qrdx * (re - rw), gyh = qrdy * (rn - rs);
-  UV(ou, 0, 0) = u;
-  UV(ou, 1, 0) = v;
-  NQ_(oq, Q_P, 0) = k.c3cv * cp * w - 3.0 * (r * r);
-  NQ_(oq, Q_TCL, 0) = ir * w;
-  NQ_(oq, Q_CP, 0) = cp;
-  NQ_(oq, Q_TCAP, 0) = 2.0 * ir * (gxh * gxh + gyh * gyh);
-  NQ_(oq, Q_LAPH, 0) = hrdx2 * ((rw - 2.0 * r) + re) + hrdy2 * ((rs - 2.0 * r) + rn);
-  NQ_(oq, Q_GXH, 0) = gxh;
-  NQ_(oq, Q_GYH, 0) = gyh;
-}
-
-// x-face between columns x-1 and x of row y: s0 = state row y, um/u0/up =
-// velocity rows y-1, y, y+1, q0 = node row y
-template <bool WALL>
-__device__ __forceinline__ void x_face(const StageArgs& a, int s0, int um, int u0, int up, int q0,
-                                       int x, double F[4]) {
-  const DimConst& k = a.k;
-  FaceIn fi;
-  fi.ra = ST(s0, 0, 1); fi.rb = ST(s0, 0, 2);
-  fi.mna = ST(s0, 1, 1); fi.mnb = ST(s0, 1, 2);
-  fi.mta = ST(s0, 2, 1); fi.mtb = ST(s0, 2, 2);
-  fi.ea = ST(s0, 3, 1); fi.eb = ST(s0, 3, 2);
-  fi.una = UV(u0, 0, 0); fi.unb = UV(u0, 0, 1);
-  fi.uta = UV(u0, 1, 0); fi.utb = UV(u0, 1, 1);
-  fi.pa = NQ_(q0, Q_P, 0); fi.pb = NQ_(q0, Q_P, 1);
-  fi.ta = NQ_(q0, Q_TCL, 0); fi.tb = NQ_(q0, Q_TCL, 1);
-  fi.ca = NQ_(q0, Q_CP, 0); fi.cb = NQ_(q0, Q_CP, 1);
-  fi.ka = NQ_(q0, Q_TCAP, 0); fi.kb = NQ_(q0, Q_TCAP, 1);
-  const double rdx = a.rdx, q_rdy = 0.25 * a.rdy;
-  fi.drn = rdx * (fi.rb - fi.ra);
-  fi.drt = NQ_(q0, Q_GYH, 0) + NQ_(q0, Q_GYH, 1);
-  fi.dunn = rdx * (fi.unb - fi.una);
-  fi.dunt = q_rdy * ((UV(up, 0, 0) + UV(up, 0, 1)) - (UV(um, 0, 0) + UV(um, 0, 1)));
-  fi.dutn = rdx * (fi.utb - fi.uta);
-  fi.dutt = q_rdy * ((UV(up, 1, 0) + UV(up, 1, 1)) - (UV(um, 1, 0) + UV(um, 1, 1)));
-  fi.lap = NQ_(q0, Q_LAPH, 0) + NQ_(q0, Q_LAPH, 1);
-  fi.dtn = rdx * (fi.tb - fi.ta);
-  fi.dkn = rdx * (fi.kb - fi.ka);
-  const bool w_face = WALL && a.wall_w && x == BC;
-  const bool e_face = WALL && a.wall_e && x == a.f.nx - BC;
-  if (w_face || e_face) {
-    const int dc = w_face ? 1 : 0;
-    const double tl = k.c38cv * (NQ_(q0, Q_TCL, dc) - k.iwe * NQ_(q0, Q_TCAP, dc));
-    const double q = wall_heat_flux(a.wall, a.xmap0 + x * a.dx);
-    wall_face_flux(fi, tl, a.dx, q, w_face ? q : -q, k, F);
-  } else {
-    face_flux(fi, k, F);
+  // the row at distance d (in u^n) into the ring row at `to`
+  __device__ __forceinline__ void un(const Field& f, ptrdiff_t d, double* to) const {
+    cp_async16(to + dst, src + d);
+    cp_async16(to + dst + 2 * RC, src + d + 2 * f.plane);
   }
-}
-
-// y-face between rows yb and yb+1 of column x: sb/st = state rows yb, yb+1,
-// ub/ut = velocity rows, qb/qt = node rows; output in conservative order
-// (mass, m_x, m_y, E)
-template <bool WALL>
-__device__ __forceinline__ void y_face(const StageArgs& a, int sb, int st, int ub, int ut, int qb,
-                                       int qt, int x, int yb, double G[4]) {
-  const DimConst& k = a.k;
-  const int yt = yb + 1;
-  FaceIn fi;
-  fi.ra = ST(sb, 0, 2); fi.rb = ST(st, 0, 2);
-  fi.mna = ST(sb, 2, 2); fi.mnb = ST(st, 2, 2);
-  fi.mta = ST(sb, 1, 2); fi.mtb = ST(st, 1, 2);
-  fi.ea = ST(sb, 3, 2); fi.eb = ST(st, 3, 2);
-  fi.una = UV(ub, 1, 1); fi.unb = UV(ut, 1, 1);
-  fi.uta = UV(ub, 0, 1); fi.utb = UV(ut, 0, 1);
-  fi.pa = NQ_(qb, Q_P, 1); fi.pb = NQ_(qt, Q_P, 1);
-  fi.ta = NQ_(qb, Q_TCL, 1); fi.tb = NQ_(qt, Q_TCL, 1);
-  fi.ca = NQ_(qb, Q_CP, 1); fi.cb = NQ_(qt, Q_CP, 1);
-  fi.ka = NQ_(qb, Q_TCAP, 1); fi.kb = NQ_(qt, Q_TCAP, 1);
-  const double rdy = a.rdy, q_rdx = 0.25 * a.rdx;
-  fi.drn = rdy * (fi.rb - fi.ra);
-  fi.drt = NQ_(qb, Q_GXH, 1) + NQ_(qt, Q_GXH, 1);
-  fi.dunn = rdy * (fi.unb - fi.una);
-  fi.dunt = q_rdx * ((UV(ub, 1, 2) + UV(ut, 1, 2)) - (UV(ub, 1, 0) + UV(ut, 1, 0)));
-  fi.dutn = rdy * (fi.utb - fi.uta);
-  fi.dutt = q_rdx * ((UV(ub, 0, 2) + UV(ut, 0, 2)) - (UV(ub, 0, 0) + UV(ut, 0, 0)));
-  fi.lap = NQ_(qb, Q_LAPH, 1) + NQ_(qt, Q_LAPH, 1);
-  fi.dtn = rdy * (fi.tb - fi.ta);
-  fi.dkn = rdy * (fi.kb - fi.ka);
-  double F[4];
-  const bool s_face = WALL && a.wall_s && yt == BC;
-  const bool n_face = WALL && a.wall_n && yt == a.f.ny - BC;
-  if (s_face || n_face) {
-    const int qo = s_face ? qt : qb;
-    const double tl = k.c38cv * (NQ_(qo, Q_TCL, 1) - k.iwe * NQ_(qo, Q_TCAP, 1));
-    const double q = wall_heat_flux(a.wall, a.xmap0 + x * a.dx);
-    wall_face_flux(fi, tl, a.dy, q, s_face ? q : -q, k, F);
-  } else {
-    face_flux(fi, k, F);
-  }
-  G[0] = F[0];
-  G[1] = F[2];  // momentum_x is tangential on a y-face
-  G[2] = F[1];
-  G[3] = F[3];
-}
-
-// ---- mixed precision (DIM2D_MIXED) -----------------------------------
-// The node pass runs in FP64 -- the van der Waals inversion for u, v, P,
-// Tcl, 1/(3-rho) and Tcap -- and stores FP32 copies of rho, m_x, m_y, E
-// and of those quantities; the face pass (stencils and flux formulas)
-// reads the FP32 copies and runs in FP32.  Tcap stays FP64 and its normal
-// derivative, the third-derivative capillary term of the energy flux, is
-// added to the face's energy flux in FP64.  Divergence and RK update are
-// FP64 on the FP64 state.
-enum NodeF : int {
-  F_R = 0, F_MX, F_MY, F_E, F_U, F_V, F_P, F_TCL, F_CP, F_LAPH, F_GXH, F_GYH, NQF
 };
-constexpr int NM = 3;              // node rows (y-1 .. y+1)
-constexpr int F_ROW = NQF * PC;    // floats per node row
-// Mixed precision keeps one u^n row (FP64 keeps two, alternating): the next
-// row's u^n is copied once the update has read this one, in its own
-// cp.async group, and waited for just before the next update.  10.8 KB per
-// warp then fits 20 warps per SM (shape 16x4x5, 96 registers).
-constexpr int WARP_DOUBLES_MIX = NS * ST_ROW + NM * PC + (NM * F_ROW + 1) / 2 + UN_ROW;
-#define FQ(o, c, dc) reinterpret_cast<float*>(g_ring)[(o) + (c) * PC + (dc)]
-#define KQ(o, dc) g_ring[(o) + (dc)]
 
-// node quantities of column c0-1+lane of one row (as node_row) into the
-// float row fo and the FP64 Tcap row ko
-__device__ __forceinline__ void node_row_mix(int sm, int s0, int sp, int fo, int ko, double qrdx,
-                                             double qrdy, double hrdx2, double hrdy2,
-                                             const DimConst& k) {
-  const double r = ST(s0, 0, 1);
-  const double rw = ST(s0, 0, 0), re = ST(s0, 0, 2);
-  const double rs = ST(sm, 0, 1), rn = ST(sp, 0, 1);
-  const double mx = ST(s0, 1, 1), my = ST(s0, 2, 1), e = ST(s0, 3, 1);
+// Products that are added to something are written as fma, and products that
+// must not be contracted as mul(), so that every instantiation of this code
+// (one field, batch, persistent kernel) rounds alike.
+__device__ __forceinline__ double mul(double a, double b) { return __dmul_rn(a, b); }
+__device__ __forceinline__ float mul(float a, float b) { return __fmul_rn(a, b); }
+
+// Node quantities of one row in the lane's column.  T = double, or float for
+// the face pass of the mixed-precision path; u, v, P, Tcl, 1/(3-rho) and
+// Tcap are always evaluated in FP64.
+template <typename T>
+struct NodeQ {
+  T r, mx, my, e;  // conservative values
+  T u, v, p;       // velocity, pressure
+  T qyy, qxy, hv;  // my v + P, mx v (= my u), (E + P) v
+  T cp;            // 1.5/cv_r / (3 - rho)
+  T lap;           // 1/We times half the density Laplacian
+  T gx, gy;        // sqrt(1/We) times half the centred density gradient
+  T dw;            // rho(x) - rho(x-1)
+  double th;       // Tcl - Tcap/We, FP64 also in mixed precision
+};
+
+// Primitives as node_prim() (dim2d_prim_module.f:242-289, 425-453, 515-544,
+// 1056-1071) with 1/rho and 1/(3-rho) from one division; Tcap = 0.5/rho
+// |grad rho|^2 with centred gradients (:582-613).  First part: what the
+// x-face of the row below takes from this row.
+// 1/d from the hardware's approximation (20 bits or better) and one step of
+// Halley's iteration, x (1 + e + e^2) with e = 1 - d x: cubic, so that the
+// remaining error is rounding (2^-60 before it).
+__device__ __forceinline__ double reciprocal(double d) {
+  double x;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(x) : "d"(d));
+  const double e = fma(-d, x, 1.0);
+  return fma(fma(e, e, e), x, x);
+}
+struct NodeUV {
+  double inv, ir, u, v;
+};
+__device__ __forceinline__ NodeUV node_uv(double r, double mx, double my) {
+  NodeUV n;
   const double tm = 3.0 - r;
-  const double inv = 1.0 / (r * tm);
-  const double ir = tm * inv;
-  const double cp = r * inv;
-  const double u = mx * ir, v = my * ir;
-  const double w = e - 0.5 * r * (u * u + v * v) + 3.0 * (r * r);
-  const double gxh = qrdx * (re - rw), gyh = qrdy * (rn - rs);
-  FQ(fo, F_R, 0) = (float)r;
-  FQ(fo, F_MX, 0) = (float)mx;
-  FQ(fo, F_MY, 0) = (float)my;
-  FQ(fo, F_E, 0) = (float)e;
-  FQ(fo, F_U, 0) = (float)u;
-  FQ(fo, F_V, 0) = (float)v;
-  FQ(fo, F_P, 0) = (float)(k.c3cv * cp * w - 3.0 * (r * r));
-  FQ(fo, F_TCL, 0) = (float)(ir * w);
-  FQ(fo, F_CP, 0) = (float)cp;
-  FQ(fo, F_LAPH, 0) = (float)(hrdx2 * ((rw - 2.0 * r) + re) + hrdy2 * ((rs - 2.0 * r) + rn));
-  FQ(fo, F_GXH, 0) = (float)gxh;
-  FQ(fo, F_GYH, 0) = (float)gyh;
-  KQ(ko, 0) = 2.0 * ir * (gxh * gxh + gyh * gyh);
+  n.inv = reciprocal(r * tm);
+  n.ir = tm * n.inv;
+  n.u = mul(mx, n.ir);
+  n.v = mul(my, n.ir);
+  return n;
+}
+// the rest; dw, de, ds, dn = density differences to the west (r - r_w), east
+// (r_e - r), south and north node
+template <typename T>
+__device__ __forceinline__ NodeQ<T> node(const NodeUV& n, double r, double mx, double my,
+                                         double e, double dw, double de, double ds, double dn,
+                                         const StripCoef<double>& c) {
+  const double cp = mul(c.c15cv * r, n.inv);
+  const double m3r2 = mul(-3.0 * r, r);
+  // W = E - rho|u|^2/2 + 3 rho^2
+  const double w = fma(-0.5, fma(mx, n.u, my * n.v), e) - m3r2;
+  const double p = fma(cp, w + w, m3r2);
+  const double gx = mul(c.gx, de + dw), gy = mul(c.gy, dn + ds);
+  NodeQ<T> q;
+  q.th = mul(n.ir, fma(-2.0, fma(gx, gx, gy * gy), w));
+  q.lap = (T)fma(c.lx, de - dw, c.ly * (dn - ds));
+  q.r = (T)r;
+  q.mx = (T)mx;
+  q.my = (T)my;
+  q.e = (T)e;
+  q.u = (T)n.u;
+  q.v = (T)n.v;
+  q.p = (T)p;
+  q.qyy = fma(q.my, q.v, q.p);
+  q.qxy = mul(q.mx, q.v);
+  q.hv = mul(q.e + q.p, q.v);
+  q.cp = (T)cp;
+  q.gx = (T)gx;
+  q.gy = (T)gy;
+  q.dw = (T)dw;
+  return q;
 }
 
-// FP64 face inputs a wall face flux reads, from the FP32 face inputs
-__device__ __forceinline__ FaceIn wall_face_in(const FaceInT<float>& fi) {
-  FaceIn d{};
-  d.ra = fi.ra;
-  d.rb = fi.rb;
-  d.drn = fi.drn;
-  d.drt = fi.drt;
-  d.dutn = fi.dutn;
-  d.lap = fi.lap;
-  return d;
+// the face pass's type and coefficients
+template <bool MIX>
+struct FaceType {
+  using type = double;
+};
+template <>
+struct FaceType<true> {
+  using type = float;
+};
+__device__ __forceinline__ const StripCoef<double>& coef_of(const StageArgs& a, double) { return a.c; }
+__device__ __forceinline__ const StripCoef<float>& coef_of(const StageArgs& a, float) { return a.cf; }
+
+// Sums (s..) and differences (d..) of the two nodes' quantities at a face,
+// in the face frame (n = normal, t = tangential).
+template <typename T>
+struct FaceSums {
+  T smn, sqn, sqt;       // m_n, m_n u_n + P, m_t u_n
+  double sh;             // (E + P) u_n - 2/(Re Pr) d/dn (Tcl - Tcap/We)
+  T scp, scu;            // cp, cp u_n
+  T sr, sun, sut;        // rho, u_n, u_t
+  T dr, dun, dut;        // normal differences
+  T gt;                  // scaled tangential density gradient
+  T dunt, dutt;          // undivided tangential differences of u_n, u_t
+  T lap;                 // Laplacian / We
+};
+
+// Twice the face flux of (mass, normal momentum, tangential momentum,
+// energy); formulas of face_flux_t (dim2d_fluxes_module.f:103-541) on sums
+// instead of averages.  tnn, tnt: viscous stress plus the capillary terms
+// that enter the energy flux with the same velocity.
+// The temperature term of the energy flux, which holds the third
+// derivatives of the capillary part, is FP64 in mixed precision too (cth).
+template <typename T>
+__device__ __forceinline__ void face2(const FaceSums<T>& f, const FaceCoef<T>& c, T s, T F[3],
+                                      double* F3) {
+  const T drn = c.s * f.dr;
+  const T drn2 = mul(drn, drn);
+  const T t = fma(f.gt, f.gt, -drn2);
+  const T g2 = fma(f.gt, f.gt, drn2);
+  const T div = fma(c.dn, f.dun, c.dt * f.dutt);
+  const T tnn = fma(T(0.5), t, fma(c.a1, f.dun, c.a2 * f.dutt));
+  const T tnt = fma(-drn, f.gt, fma(c.b1, f.dunt, c.b2 * f.dut));
+  F[0] = f.smn;
+  F[1] = fma(T(-2), tnn, f.sqn) - fma(f.scp, g2, f.sr * f.lap);
+  F[2] = fma(T(-2), tnt, f.sqt);
+  const T cap = fma(-(f.sr * (s * drn)), div, fma(f.scu, g2, f.smn * f.lap));
+  *F3 = f.sh - (double)fma(f.sun, tnn, fma(f.sut, tnt, cap));
 }
 
-// x-face between columns x-1 and x of row y: fm/f0/fp = node rows y-1, y,
-// y+1, k0 = Tcap row y
-template <bool WALL>
-__device__ __forceinline__ void x_face_mix(const StageArgs& a, const FluxCoefF& kf, int fm, int f0,
-                                           int fp, int k0, int x, double F[4]) {
-  const DimConst& k = a.k;
-  FaceInT<float> fi;
-  fi.ra = FQ(f0, F_R, 0); fi.rb = FQ(f0, F_R, 1);
-  fi.mna = FQ(f0, F_MX, 0); fi.mnb = FQ(f0, F_MX, 1);
-  fi.mta = FQ(f0, F_MY, 0); fi.mtb = FQ(f0, F_MY, 1);
-  fi.ea = FQ(f0, F_E, 0); fi.eb = FQ(f0, F_E, 1);
-  fi.una = FQ(f0, F_U, 0); fi.unb = FQ(f0, F_U, 1);
-  fi.uta = FQ(f0, F_V, 0); fi.utb = FQ(f0, F_V, 1);
-  fi.pa = FQ(f0, F_P, 0); fi.pb = FQ(f0, F_P, 1);
-  fi.ta = FQ(f0, F_TCL, 0); fi.tb = FQ(f0, F_TCL, 1);
-  fi.ca = FQ(f0, F_CP, 0); fi.cb = FQ(f0, F_CP, 1);
-  fi.ka = fi.kb = 0.0f;
-  const float rdx = (float)a.rdx, q_rdy = 0.25f * (float)a.rdy;
-  fi.drn = rdx * (fi.rb - fi.ra);
-  fi.drt = FQ(f0, F_GYH, 0) + FQ(f0, F_GYH, 1);
-  fi.dunn = rdx * (fi.unb - fi.una);
-  fi.dunt = q_rdy * ((FQ(fp, F_U, 0) + FQ(fp, F_U, 1)) - (FQ(fm, F_U, 0) + FQ(fm, F_U, 1)));
-  fi.dutn = rdx * (fi.utb - fi.uta);
-  fi.dutt = q_rdy * ((FQ(fp, F_V, 0) + FQ(fp, F_V, 1)) - (FQ(fm, F_V, 0) + FQ(fm, F_V, 1)));
-  fi.lap = FQ(f0, F_LAPH, 0) + FQ(f0, F_LAPH, 1);
-  fi.dtn = rdx * (fi.tb - fi.ta);
-  fi.dkn = 0.0f;
-  const bool w_face = WALL && a.wall_w && x == BC;
-  const bool e_face = WALL && a.wall_e && x == a.f.nx - BC;
-  if (w_face || e_face) {
-    const int dc = w_face ? 1 : 0;
-    const double tl = k.c38cv * ((double)FQ(f0, F_TCL, dc) - k.iwe * KQ(k0, dc));
-    const double q = wall_heat_flux(a.wall, a.xmap0 + x * a.dx);
-    wall_face_flux(wall_face_in(fi), tl, a.dx, q, w_face ? q : -q, k, F);
-    return;
-  }
-  float Ff[4];
-  face_flux_t<float, FluxCoefF, false>(fi, kf, Ff);
-#pragma unroll
-  for (int v = 0; v < 4; v++) F[v] = (double)Ff[v];
-  // -(1/We) * (-(1/(Re Pr)) dTcap/dn), FP64
-  F[3] += k.iwe * k.irepr * (a.rdx * (KQ(k0, 1) - KQ(k0, 0)));
+// Twice the flux of the south wall's face (wall_face_flux,
+// wall_xy_equilibrium_module.f:445-908): th = Tcl - Tcap/We of the first
+// interior node, q = wall heat flux.
+template <typename T>
+__device__ __forceinline__ void wall_face2(const FaceSums<T>& f, const FaceCoef<T>& c, double th,
+                                           double dy, double q, const DimConst& k, T F[3],
+                                           double* F3) {
+  const double tl = k.c38cv * th;
+  const double t_half = 0.5 * (tl + (tl + dy * k.c38cv * k.re * k.pr * q));
+  const double md = 0.5 * (double)f.sr, drn = (double)(c.s * f.dr), gt = (double)f.gt;
+  const double p = 8.0 * md * t_half / (3.0 - md) - 3.0 * (md * md);
+  F[0] = T(0);
+  F[1] = (T)(2.0 * p - ((double)(f.sr * f.lap) + (gt * gt - drn * drn)));
+  F[2] = (T)(-2.0 * ((double)(c.b2 * f.dut) - drn * gt));
+  *F3 = 2.0 * q;
 }
 
-// y-face between rows yb and yb+1 of column x: fb/ft = node rows yb, yb+1,
-// kb/kt = their Tcap rows; output in conservative order
-template <bool WALL>
-__device__ __forceinline__ void y_face_mix(const StageArgs& a, const FluxCoefF& kf, int fb, int ft,
-                                           int kb, int kt, int x, int yb, double G[4]) {
-  const DimConst& k = a.k;
-  const int yt = yb + 1;
-  FaceInT<float> fi;
-  fi.ra = FQ(fb, F_R, 1); fi.rb = FQ(ft, F_R, 1);
-  fi.mna = FQ(fb, F_MY, 1); fi.mnb = FQ(ft, F_MY, 1);
-  fi.mta = FQ(fb, F_MX, 1); fi.mtb = FQ(ft, F_MX, 1);
-  fi.ea = FQ(fb, F_E, 1); fi.eb = FQ(ft, F_E, 1);
-  fi.una = FQ(fb, F_V, 1); fi.unb = FQ(ft, F_V, 1);
-  fi.uta = FQ(fb, F_U, 1); fi.utb = FQ(ft, F_U, 1);
-  fi.pa = FQ(fb, F_P, 1); fi.pb = FQ(ft, F_P, 1);
-  fi.ta = FQ(fb, F_TCL, 1); fi.tb = FQ(ft, F_TCL, 1);
-  fi.ca = FQ(fb, F_CP, 1); fi.cb = FQ(ft, F_CP, 1);
-  fi.ka = fi.kb = 0.0f;
-  const float rdy = (float)a.rdy, q_rdx = 0.25f * (float)a.rdx;
-  fi.drn = rdy * (fi.rb - fi.ra);
-  fi.drt = FQ(fb, F_GXH, 1) + FQ(ft, F_GXH, 1);
-  fi.dunn = rdy * (fi.unb - fi.una);
-  fi.dunt = q_rdx * ((FQ(fb, F_V, 2) + FQ(ft, F_V, 2)) - (FQ(fb, F_V, 0) + FQ(ft, F_V, 0)));
-  fi.dutn = rdy * (fi.utb - fi.uta);
-  fi.dutt = q_rdx * ((FQ(fb, F_U, 2) + FQ(ft, F_U, 2)) - (FQ(fb, F_U, 0) + FQ(ft, F_U, 0)));
-  fi.lap = FQ(fb, F_LAPH, 1) + FQ(ft, F_LAPH, 1);
-  fi.dtn = rdy * (fi.tb - fi.ta);
-  fi.dkn = 0.0f;
-  double F[4];
-  const bool s_face = WALL && a.wall_s && yt == BC;
-  const bool n_face = WALL && a.wall_n && yt == a.f.ny - BC;
-  if (s_face || n_face) {
-    const int fo = s_face ? ft : fb, ko = s_face ? kt : kb;
-    const double tl = k.c38cv * ((double)FQ(fo, F_TCL, 1) - k.iwe * KQ(ko, 1));
-    const double q = wall_heat_flux(a.wall, a.xmap0 + x * a.dx);
-    wall_face_flux(wall_face_in(fi), tl, a.dy, q, s_face ? q : -q, k, F);
-  } else {
-    float Ff[4];
-    face_flux_t<float, FluxCoefF, false>(fi, kf, Ff);
-#pragma unroll
-    for (int v = 0; v < 4; v++) F[v] = (double)Ff[v];
-    F[3] += k.iwe * k.irepr * (a.rdy * (KQ(kt, 1) - KQ(kb, 1)));
-  }
-  G[0] = F[0];
-  G[1] = F[2];
-  G[2] = F[1];
-  G[3] = F[3];
+// x-face between the lane's column and the one to the left, row y: n = node
+// quantities of row y, ul, vl = the left column's velocity, gyu, gyv =
+// undivided velocity differences across row y
+template <typename T>
+__device__ __forceinline__ void x_face(const NodeQ<T>& n, T ul, T vl, T gyu, T gyv,
+                                       const StripCoef<T>& c, double cth, T F[3], double* F3) {
+  FaceSums<T> f;
+  const T cl = from_left(n.cp);
+  f.smn = from_left(n.mx) + n.mx;
+  const T qxx = fma(n.mx, n.u, n.p), hu = mul(n.e + n.p, n.u);
+  f.sqn = from_left(qxx) + qxx;
+  f.sqt = from_left(n.qxy) + n.qxy;
+  if (sizeof(T) == sizeof(double))  // the low side's term travels whole: one exchange
+    f.sh = from_left(fma(cth, n.th, (double)hu)) + fma(-cth, n.th, (double)hu);
+  else
+    f.sh = fma(-cth, n.th - from_left(n.th), (double)(from_left(hu) + hu));
+  f.scp = cl + n.cp;
+  f.scu = fma(cl, ul, n.cp * n.u);
+  f.sr = fma(T(2), n.r, -n.dw);
+  f.sun = ul + n.u;
+  f.sut = vl + n.v;
+  f.dr = n.dw;
+  f.dun = n.u - ul;
+  f.dut = n.v - vl;
+  f.gt = from_left(n.gy) + n.gy;
+  f.dunt = from_left(gyu) + gyu;
+  f.dutt = from_left(gyv) + gyv;
+  f.lap = from_left(n.lap) + n.lap;
+  face2(f, c.x, c.s, F, F3);
 }
 
-// boundary kinds of the strip kernel
-// K_WALL_OPEN: open sections and a south wall (wall_S_open,
-// half_wall_S_open): ghost CTAs of the open sections, wall faces in the strips
-enum StripKind : int { K_PLAIN = 0, K_WALL = 1, K_OPEN = 2, K_WALL_OPEN = 3 };
+// y-face between rows y (b) and y+1 (t) of the lane's column: dr = density
+// difference, g..u, g..v = undivided velocity differences across the column
+template <typename T>
+__device__ __forceinline__ FaceSums<T> y_sums(const NodeQ<T>& b, const NodeQ<T>& t, T dr, T gxub,
+                                              T gxut, T gxvb, T gxvt, double cth) {
+  FaceSums<T> f;
+  f.smn = b.my + t.my;
+  f.sqn = b.qyy + t.qyy;
+  f.sqt = b.qxy + t.qxy;
+  f.sh = fma(-cth, t.th - b.th, (double)(b.hv + t.hv));
+  f.scp = b.cp + t.cp;
+  f.scu = fma(b.cp, b.v, t.cp * t.v);
+  f.sr = b.r + t.r;
+  f.sun = b.v + t.v;
+  f.sut = b.u + t.u;
+  f.dr = dr;
+  f.dun = t.v - b.v;
+  f.dut = t.u - b.u;
+  f.gt = b.gx + t.gx;
+  f.dunt = gxvb + gxvt;
+  f.dutt = gxub + gxut;
+  f.lap = b.lap + t.lap;
+  return f;
+}
 
 // The strip of one warp: columns c0 .. c0+29 (interior ones), rows y0 ..
-// y1-1, with ring slot `warp` of the CTA's shared memory.
-template <int MODE, bool WALL, bool MIX>
-__device__ __forceinline__ void strip_warp(const StageArgs& a, int c0, int y0, int y1, int warp) {
+// y1-1.
+// UN: whether the stage reads u^n (stages 2 and 3), 2: by a.stage.
+template <int MODE, int UN, bool MIX>
+__device__ __forceinline__ void strip_warp(const StageArgs& a, int c0, int y0, int y1) {
+  using T = typename FaceType<MIX>::type;
   const int lane = threadIdx.x & 31;
   const Field f = a.f;
-  const int x = c0 + lane;
-  const DimConst& k = a.k;
-  const double qrdx = 0.25 * a.rdx, qrdy = 0.25 * a.rdy;
-  const double hrdx2 = 0.5 * a.rdx * a.rdx, hrdy2 = 0.5 * a.rdy * a.rdy;
-  const bool need_un = MODE == 1 && a.stage != 1;
-
-  // ring row offsets (warp base + lane column)
-  const int wbase = warp * (MIX ? WARP_DOUBLES_MIX : WARP_DOUBLES);
-  const int wb = wbase + lane;
-  int s0 = wb, s1 = wb + ST_ROW, s2 = wb + 2 * ST_ROW, s3 = wb + 3 * ST_ROW;  // state rows
-  const int ub = wb + NS * ST_ROW;
-  int um = ub, u0 = ub + UV_ROW, u1 = ub + 2 * UV_ROW;  // velocity rows
-  const int qbase = ub + NUV * UV_ROW;
-  int q0 = qbase, q1 = qbase + Q_ROW;                   // node rows
-  // mixed precision: Tcap rows (doubles) and FP32 node rows (floats)
-  int km = ub, k0 = ub + PC, k1 = ub + 2 * PC;
-  const int fbase = 2 * (wbase + NS * ST_ROW + NM * PC) + lane;
-  int fm = fbase, f0 = fbase + F_ROW, f1 = fbase + 2 * F_ROW;
-  const FluxCoefF kf = flux_coef_f32(k);
-  // u^n rows (two, alternating), after the rest of the warp's region
-  const int unb = wbase + (MIX ? NS * ST_ROW + NM * PC + (NM * F_ROW + 1) / 2
-                               : NS * ST_ROW + NUV * UV_ROW + NQ * Q_ROW) + lane;
-  int un0 = unb, un1 = MIX ? unb : unb + UN_ROW;
+  const StripCoef<double>& cd = a.c;
+  const StripCoef<T>& c = coef_of(a, T(0));
+  const bool need_un = MODE == 1 && (UN == 2 ? a.stage != 1 : UN == 1);
 
   if (a.node_sides && reads_node_ghosts(a.node_sides, f, c0, y0, y1)) wait_for_node_pass();
 
-  // prologue: state rows y0-2, y0-1, y0, y0+1 (s3, s2, s0, s1), all four
-  // copies in flight together; node quantities of rows y0-1 (um, q1) and
-  // y0 (u0, q0); bottom face of row y0; then row y0+2 (into s2) and u^n of
-  // row y0 on their way
-  async_row(a, c0, y0 - 2, lane, s3);
-  async_row(a, c0, y0 - 1, lane, s2);
-  async_row(a, c0, y0, lane, s0);
-  async_row(a, c0, y0 + 1, lane, s1);
-  cp_async_commit();
-  cp_async_wait<0>();
-  __syncwarp();
-  if (MIX) {
-    node_row_mix(s3, s2, s0, fm, km, qrdx, qrdy, hrdx2, hrdy2, k);
-    node_row_mix(s2, s0, s1, f0, k0, qrdx, qrdy, hrdx2, hrdy2, k);
-  } else {
-    node_row(s3, s2, s0, um, q1, qrdx, qrdy, hrdx2, hrdy2, k);
-    node_row(s2, s0, s1, u0, q0, qrdx, qrdy, hrdx2, hrdy2, k);
-  }
-  __syncwarp();
-  double Gb[4];
-  if (MIX) y_face_mix<WALL>(a, kf, fm, f0, km, k0, x, y0 - 1, Gb);
-  else y_face<WALL>(a, s2, s0, um, u0, q1, q0, x, y0 - 1, Gb);
-  __syncwarp();  // rows y0-2 and y0-1 are no longer read
-  async_row(a, c0, y0 + 2, lane, s2);
-  if (MIX) cp_async_commit();  // mixed: u^n rows travel in their own groups
-  if (need_un) async_un(a, c0, y0, un0, lane);
-  cp_async_commit();
+  // the lane's column (columns past the field are not stored); its place in
+  // a ring row
+  const int x = c0 - 1 + lane;
+  const size_t P = f.pitch, V = f.plane;
+  double* const ring = g_ring + (threadIdx.x >> 5) * WARP_DOUBLES;
+  double* const uring = ring + NS * ST_ROW;
+  auto st = [&](int slot) { return ring + slot * ST_ROW + lane + 1; };
 
-  const bool active = lane < SW && x <= f.nx - 1 - BC &&
+  // rows y0-2 .. y0+2 into slots 0 .. 4, all in flight together
+  RowCopy copy(a.uin, f, c0, y0 - 2, lane);
+#pragma unroll
+  for (int i = 0; i < 4; i++) {
+    copy.state(f, ring + i * ST_ROW, lane);
+    copy.src += P;
+  }
+  cp_async_commit();
+  // u^n of the row two below the state row being copied
+  const ptrdiff_t un_row = (a.u0 - a.uin) - 2 * (ptrdiff_t)P;
+  copy.state(f, ring + 4 * ST_ROW, lane);
+  if (need_un) copy.un(f, un_row, uring);
+  copy.src += P;
+  cp_async_commit();
+  cp_async_wait<1>();
+  __syncwarp();
+  const double rm = st(1)[0];
+  double r0 = st(2)[0], mx0 = st(2)[RC], my0 = st(2)[2 * RC], e0 = st(2)[3 * RC];
+  double r1 = st(3)[0];
+
+  // node quantities of rows y0-1 and y0, bottom face of row y0
+  NodeQ<T> n0;
+  T um, vm;              // velocity of row y-1
+  T ul0, vl0, gxu0, gxv0;  // row y: left velocity, undivided differences across the column
+  double dn0 = r1 - r0;  // density difference between rows y and y+1
+  T Gb[3];  // in the face frame: mass, m_y, m_x
+  double gb3;
+  {
+    const double dn = r0 - rm;
+    const double mxm = st(1)[RC], mym = st(1)[2 * RC];
+    const NodeQ<T> nm = node<T>(node_uv(rm, mxm, mym), rm, mxm, mym, st(1)[3 * RC],
+                                rm - st(1)[-1], st(1)[1] - rm, rm - st(0)[0], dn, cd);
+    n0 = node<T>(node_uv(r0, mx0, my0), r0, mx0, my0, e0, r0 - st(2)[-1], st(2)[1] - r0, dn, dn0,
+                 cd);
+    um = nm.u;
+    vm = nm.v;
+    ul0 = from_left(n0.u);
+    vl0 = from_left(n0.v);
+    gxu0 = from_right(n0.u) - ul0;
+    gxv0 = from_right(n0.v) - vl0;
+    const FaceSums<T> s = y_sums(nm, n0, (T)dn, (T)(from_right(um) - from_left(um)), gxu0,
+                                 (T)(from_right(vm) - from_left(vm)), gxv0, cd.y.th);
+    if (a.wall_s && y0 == BC)
+      wall_face2(s, c.y, n0.th, a.dy, wall_heat_flux(a.wall, a.xmap0 + x * a.dx), a.k, Gb, &gb3);
+    else
+      face2(s, c.y, c.s, Gb, &gb3);
+  }
+
+  const bool active = lane >= 1 && lane <= SW && x <= f.nx - 1 - BC &&
                       (MODE != 2 || (x >= a.box_x0 && x <= a.box_x1));
   int ix2 = -1;
-  if (a.periodic) {
+  if (MODE == 1 && a.periodic) {
     const int px = f.nx - 2 * BC;
     if (x < 2 * BC) ix2 = x + px;
     else if (x >= f.nx - 2 * BC) ix2 = x - px;
   }
+  // stage update: out = b u^n + (1 - b) (u + dt L), L from doubled fluxes
+  const double w = MODE == 1 ? (1.0 - a.b) * a.dt : 1.0;
+  const double wx = 0.5 * a.rdx * w, wy = 0.5 * a.rdy * w;
 
-  // s0/s1/s2 = state rows y, y+1, y+2 (row y+2 may still be landing), s3
-  // the free slot; un0 = u^n of row y (may be landing), un1 free; um/u0 =
-  // velocity rows y-1, y and u1 free; q0 = node row y and q1 free
-#pragma unroll 1
+  double* __restrict__ out = a.uout + (size_t)y0 * P + x;
+
+  const double* const un = uring + lane + 1;
+
+  // the next row's copies: state row y0+3 into the slot of row y0-2
+  __syncwarp();
+  if (y0 + 1 < y1) {
+    copy.state(f, ring, lane);
+    if (need_un) copy.un(f, un_row, uring + UN_ROW);
+    copy.src += P;
+  }
+  cp_async_commit();
+
+  // ring slots of state rows y+1, y+2 and (to be written) y+4, of u^n rows y
+  // and (to be written) y+2
+  int o1 = 3 * ST_ROW, o2 = 4 * ST_ROW, ow = ST_ROW, ou = 0, ouw = 2 * UN_ROW;
+
+  // r0/mx0/my0/e0 = state row y, r1 = density of row y+1
+#pragma unroll 2
   for (int y = y0; y < y1; y++) {
-    async_row(a, c0, y + 3, lane, s3);  // next row: lands during this one
-    if (!MIX && need_un) async_un(a, c0, y + 1, un1, lane);
+    if (y + 2 < y1) {
+      copy.state(f, ring + ow, lane);
+      if (need_un) copy.un(f, un_row, uring + ouw);
+      copy.src += P;
+    }
     cp_async_commit();
-    // FP64: all but the group just issued (rows y+2, u^n(y)); mixed: all
-    // but that one and u^n(y)'s, which is waited for before the update
-    if (MIX) cp_async_wait<2>();
-    else cp_async_wait<1>();
+    cp_async_wait<2>();  // rows up to y+2 and u^n(y) are there
     __syncwarp();
-    if (MIX) node_row_mix(s0, s1, s2, f1, k1, qrdx, qrdy, hrdx2, hrdy2, k);
-    else node_row(s0, s1, s2, u1, q1, qrdx, qrdy, hrdx2, hrdy2, k);
-    __syncwarp();
-    double Fx[4], Gt[4];
-    if (MIX) {
-      x_face_mix<WALL>(a, kf, fm, f0, f1, k0, x, Fx);
-      y_face_mix<WALL>(a, kf, f0, f1, k0, k1, x, y, Gt);
-    } else {
-      x_face<WALL>(a, s0, um, u0, u1, q0, x, Fx);
-      y_face<WALL>(a, s0, s1, u0, u1, q0, q1, x, y, Gt);
+    const double* const s1 = ring + o1 + lane + 1;
+    const double mx1 = s1[RC], my1 = s1[2 * RC], e1 = s1[3 * RC];
+    const double r2 = ring[o2 + lane + 1];
+
+    // velocity of row y+1
+    const NodeUV uv = node_uv(r1, mx1, my1);
+    const T gyu = (T)uv.u - um, gyv = (T)uv.v - vm;
+
+    // x-face of row y, and the right one from lane+1
+    T Fx[3];
+    double fx3;
+    x_face(n0, ul0, vl0, gyu, gyv, c, cd.x.th, Fx, &fx3);
+    double D[4];  // 2 (F_left - F_right)
+#pragma unroll
+    for (int v = 0; v < 3; v++) D[v] = (double)Fx[v] - (double)from_right(Fx[v]);
+    D[3] = fx3 - from_right(fx3);
+
+    // node quantities of row y+1
+    const double dn1 = r2 - r1;
+    const NodeQ<T> n1 =
+        node<T>(uv, r1, mx1, my1, e1, r1 - s1[-1], s1[1] - r1, dn0, dn1, cd);
+
+    // y-face between rows y and y+1
+    const T ul1 = from_left(n1.u), vl1 = from_left(n1.v);
+    const T gxu1 = from_right(n1.u) - ul1, gxv1 = from_right(n1.v) - vl1;
+    T Gt[3];
+    double gt3;
+    face2(y_sums(n0, n1, (T)dn0, gxu0, gxu1, gxv0, gxv1, cd.y.th), c.y, c.s, Gt, &gt3);
+
+    // update of cell (x, y)
+    const double uc[4] = {r0, mx0, my0, e0};
+    double q[4];
+#pragma unroll
+    for (int v = 0; v < 4; v++) {
+      const int g = v == 1 ? 2 : (v == 2 ? 1 : 0);  // frame order of m_x and m_y
+      const double dG = v < 3 ? (double)Gb[g] - (double)Gt[g] : gb3 - gt3;
+      q[v] = MODE != 1 ? 0.0 : need_un ? fma(a.b, un[ou + v * RC], (1.0 - a.b) * uc[v]) : uc[v];
+      q[v] = fma(wx, D[v], fma(wy, dG, q[v]));
     }
-    double Fr[4];
-#pragma unroll
-    for (int v = 0; v < 4; v++) Fr[v] = __shfl_down_sync(0xffffffffu, Fx[v], 1);
-    if (MIX) {
-      cp_async_wait<1>();  // u^n(y)
-      __syncwarp();
+    if (a.k.gravity_ac) {  // pmodel_eq_class.f:1889-1904
+      q[2] = fma(-w, r0 * a.k.gravity, q[2]);
+      q[3] = fma(-w, my0 * a.k.gravity, q[3]);
     }
-    {
-      // every lane evaluates the update; only active lanes store
-      const size_t go = (size_t)y * f.pitch + min(x, f.nx - 1 - BC);
-      const double uc[4] = {ST(s0, 0, 2), ST(s0, 1, 2), ST(s0, 2, 2), ST(s0, 3, 2)};
-      double out[4];
+    // MODE 2 writes the interior_pt points of the layer map only
+    if (active && (MODE != 2 || __ldg(a.mask + (size_t)y * P + x) == 1)) {
 #pragma unroll
-      for (int v = 0; v < 4; v++) {
-        double L = (Fx[v] - Fr[v]) * a.rdx + (Gb[v] - Gt[v]) * a.rdy;
-        if (k.gravity_ac) {  // pmodel_eq_class.f:1889-1904
-          if (v == 2) L += -uc[0] * k.gravity;
-          if (v == 3) L += -uc[2] * k.gravity;
-        }
-        if (MODE != 1) out[v] = L;
-        else if (a.stage == 1) out[v] = uc[v] + a.dt * L;
-        else out[v] = a.b * g_ring[un0 + v * 32] + (1.0 - a.b) * (uc[v] + a.dt * L);
-      }
-      // MODE 2 writes the interior_pt points of the layer map only
-      if (active && (MODE != 2 || __ldg(a.mask + go) == 1)) {
+      for (int v = 0; v < 4; v++) out[v * V] = q[v];
+      if (MODE == 1 && a.periodic) {  // periodic_xy/bc_operators_class.f:156-199
+        int iy2 = -1;
+        const int py = f.ny - 2 * BC;
+        if (y < 2 * BC) iy2 = y + py;
+        else if (y >= f.ny - 2 * BC) iy2 = y - py;
 #pragma unroll
-        for (int v = 0; v < 4; v++) a.uout[go + v * f.plane] = out[v];
-        if (MODE == 1 && a.periodic) {  // periodic_xy/bc_operators_class.f:156-199
-          int iy2 = -1;
-          const int py = f.ny - 2 * BC;
-          if (y < 2 * BC) iy2 = y + py;
-          else if (y >= f.ny - 2 * BC) iy2 = y - py;
-#pragma unroll
-          for (int v = 0; v < 4; v++) {
-            double* dst = a.uout + v * f.plane;
-            if (ix2 >= 0) dst[(size_t)y * f.pitch + ix2] = out[v];
-            if (iy2 >= 0) {
-              dst[(size_t)iy2 * f.pitch + x] = out[v];
-              if (ix2 >= 0) dst[(size_t)iy2 * f.pitch + ix2] = out[v];
-            }
+        for (int v = 0; v < 4; v++) {
+          double* dst = a.uout + v * V;
+          if (ix2 >= 0) dst[(size_t)y * P + ix2] = q[v];
+          if (iy2 >= 0) {
+            dst[(size_t)iy2 * P + x] = q[v];
+            if (ix2 >= 0) dst[(size_t)iy2 * P + ix2] = q[v];
           }
         }
       }
     }
-#pragma unroll
-    for (int v = 0; v < 4; v++) Gb[v] = Gt[v];
-    __syncwarp();  // row y and u^n(y) are no longer read
-    if (MIX) {  // mixed: one u^n slot, refilled now that row y is done
-      if (need_un) async_un(a, c0, y + 1, un0, lane);
-      cp_async_commit();
-    }
-    const int t = s0;
-    s0 = s1;
-    s1 = s2;
-    s2 = s3;
-    s3 = t;
-    const int tn = un0;
-    un0 = un1;
-    un1 = tn;
-    const int tu = um;
-    um = u0;
-    u0 = u1;
-    u1 = tu;
-    const int tq = q0;
-    q0 = q1;
-    q1 = tq;
-    const int tf = fm;
-    fm = f0;
-    f0 = f1;
-    f1 = tf;
-    const int tk = km;
-    km = k0;
-    k0 = k1;
-    k1 = tk;
+    out += P;
+
+    um = n0.u;
+    vm = n0.v;
+    n0 = n1;
+    ul0 = ul1;
+    vl0 = vl1;
+    gxu0 = gxu1;
+    gxv0 = gxv1;
+    Gb[0] = Gt[0];
+    Gb[1] = Gt[1];
+    Gb[2] = Gt[2];
+    gb3 = gt3;
+    dn0 = dn1;
+    r0 = r1;
+    mx0 = mx1;
+    my0 = my1;
+    e0 = e1;
+    r1 = r2;
+    __syncwarp();  // row y+1 and u^n(y) have been read
+    o1 = o2;
+    o2 = o2 == (NS - 1) * ST_ROW ? 0 : o2 + ST_ROW;
+    ow = ow == (NS - 1) * ST_ROW ? 0 : ow + ST_ROW;
+    ou = ou == (NU - 1) * UN_ROW ? 0 : ou + UN_ROW;
+    ouw = ouw == (NU - 1) * UN_ROW ? 0 : ouw + UN_ROW;
   }
-  cp_async_wait<0>();  // the copies of rows past the strip land before the warp exits
+  cp_async_wait<0>();  // nothing lands after the warp's end or in its next strip
+  __syncwarp();
 }
 
-// grid: [ghost CTAs (K_OPEN only)] + sx * sy strip CTAs, x fastest
-// The work of strip CTA number b of one field (sx strips per row band).
-template <int H, int WPC, int MODE, bool WALL, bool MIX>
-__device__ __forceinline__ void strip_cta(const StageArgs& a, int b, int sx) {
-  const int warp = threadIdx.x >> 5;
+// The strip of CTA number b of one field (one warp per CTA): sx strips per
+// band of h rows, x fastest.
+template <int MODE, int UN, bool MIX>
+__device__ __forceinline__ void strip_cta(const StageArgs& a, int b, int sx, int h) {
   // MODE 2 (buffer-layer grid): strips over the border box, the first one
   // starting at an even column so that the rows' 16-byte pairs stay aligned
   const int c0 = (MODE == 2 ? (a.box_x0 & ~1) : BC) + (b % sx) * SW;
-  const int y0 = (MODE == 2 ? a.box_y0 : BC) + ((b / sx) * WPC + warp) * H;
+  const int y0 = (MODE == 2 ? a.box_y0 : BC) + (b / sx) * h;
   const int ylast = MODE == 2 ? a.box_y1 : a.f.ny - BC - 1;
-  if (y0 > ylast) return;  // the whole warp leaves; no CTA barrier is used
-  strip_warp<MODE, WALL, MIX>(a, c0, y0, min(y0 + H, ylast + 1), warp);
+  strip_warp<MODE, UN, MIX>(a, c0, y0, min(y0 + h, ylast + 1));
 }
 
-template <int H, int WPC, int MINB, int MODE, int KIND, bool MIX>
-__global__ void __launch_bounds__(32 * WPC, MINB) k_strip(StageArgs a, int ghost_ctas, int sx) {
+// grid: [ghost CTAs (OPEN only)] + strip CTAs, one warp each
+template <int MODE, int UN, bool OPEN, bool MIX>
+__global__ void __launch_bounds__(32, WARPS) k_strip(const __grid_constant__ StageArgs a,
+                                                    int ghost_ctas, int sx, int h) {
   int b = blockIdx.x;
-  if (KIND == K_OPEN || KIND == K_WALL_OPEN) {
+  if (OPEN) {
     if (b < ghost_ctas) {
       if (a.node_sides) wait_for_node_pass();  // ghost frames reach the wall rows
-      open_ghost_cell(a, b * (32 * WPC) + threadIdx.x, MODE);
+      open_ghost_cell(a, b * 32 + threadIdx.x, MODE);
       return;
     }
     b -= ghost_ctas;
   }
-  strip_cta<H, WPC, MODE, KIND == K_WALL || KIND == K_WALL_OPEN, MIX>(a, b, sx);
+  strip_cta<MODE, UN, MIX>(a, b, sx, h);
 }
 
 // stage arguments of domain i of a batched launch
+template <bool MIX>
 __device__ __forceinline__ StageArgs batch_stage_args(const BatchStageArgs& P, int i) {
   const BatchDomain& d = P.d[i];
   StageArgs a;
@@ -633,6 +594,8 @@ __device__ __forceinline__ StageArgs batch_stage_args(const BatchStageArgs& P, i
   a.ymap0 = 0.0;
   a.wall = P.wall;
   a.k = P.k;
+  a.c = d.c;
+  if (MIX) a.cf = strip_coef_f32(d.c);
   return a;
 }
 
@@ -652,24 +615,23 @@ __device__ __forceinline__ int batch_domain(const BatchStageArgs& P, int b) {
 // One RK stage of every domain of a batch (one boundary kind): the ghost
 // CTAs of all domains first (open and wall kinds: each domain's open
 // sections), then every domain's strip CTAs.
-template <int H, int WPC, int MINB, int KIND, bool MIX>
-__global__ void __launch_bounds__(32 * WPC, MINB)
-    k_strip_batch(const __grid_constant__ BatchStageArgs P) {
+template <int UN, bool OPEN, bool MIX>
+__global__ void __launch_bounds__(32, WARPS)
+    k_strip_batch(const __grid_constant__ BatchStageArgs P, int h) {
   int b = blockIdx.x;
-  if (KIND == K_OPEN || KIND == K_WALL_OPEN) {
+  if (OPEN) {
     if (b < P.ghost_ctas) {
       const int i = batch_domain<true>(P, b);
-      const StageArgs a = batch_stage_args(P, i);
+      const StageArgs a = batch_stage_args<false>(P, i);
       if (a.node_sides) wait_for_node_pass();
-      open_ghost_cell(a, (b - P.d[i].ghost0) * (32 * WPC) + threadIdx.x, 1);
+      open_ghost_cell(a, (b - P.d[i].ghost0) * 32 + threadIdx.x, 1);
       return;
     }
     b -= P.ghost_ctas;
   }
   const int i = batch_domain<false>(P, b);
-  const StageArgs a = batch_stage_args(P, i);
-  strip_cta<H, WPC, 1, KIND == K_WALL || KIND == K_WALL_OPEN, MIX>(a, b - P.d[i].strip0,
-                                                                     P.d[i].sx);
+  const StageArgs a = batch_stage_args<MIX>(P, i);
+  strip_cta<1, UN, MIX>(a, b - P.d[i].strip0, P.d[i].sx, h);
 }
 
 // ---- persistent batched kernel -----------------------------------------
@@ -720,6 +682,7 @@ __device__ bool wait_done(const PersistArgs& P, const unsigned long long* done,
   return false;
 }
 
+template <bool MIX>
 __device__ __forceinline__ StageArgs persist_stage_args(const PersistArgs& P, const PDomain& d,
                                                         int step, int st) {
   const int odd = (P.step0 + step) & 1;
@@ -751,6 +714,8 @@ __device__ __forceinline__ StageArgs persist_stage_args(const PersistArgs& P, co
   a.box_x0 = a.box_x1 = a.box_y0 = a.box_y1 = 0;
   a.wall = P.wall;
   a.k = P.k;
+  a.c = d.c;
+  if (MIX) a.cf = strip_coef_f32(d.c);
   return a;
 }
 
@@ -789,7 +754,7 @@ __device__ __forceinline__ bool wait_band(const PersistArgs& P, const PDomain& d
 
 template <bool MIX>
 __global__ void __launch_bounds__(32 * PW, 8) k_batch_persistent(const __grid_constant__ PersistArgs P) {
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int lane = threadIdx.x & 31;
   const unsigned long long total = (unsigned long long)P.items_per_step * P.nsteps;
   for (;;) {
     unsigned long long it = 0;
@@ -839,17 +804,17 @@ __global__ void __launch_bounds__(32 * PW, 8) k_batch_persistent(const __grid_co
     // a wait that ran out stops the warp (the launch is aborted)
     if (!__all_sync(0xffffffffu, ok)) break;
     if (item.type == PI_STRIP) {
-      const StageArgs a = persist_stage_args(P, d, step, item.stage);
+      const StageArgs a = persist_stage_args<MIX>(P, d, step, item.stage);
       const int c0 = BC + (item.index % d.sx) * SW;
       const int y0 = BC + item.band * P.h_rows;
       // the last band runs to the last interior row (it absorbs a remainder
       // of fewer than 2 rows, so that the rows a periodic field images into
       // the opposite ghost rows never span two bands)
       const int y1 = item.band == d.nb - 1 ? d.f.ny - BC : y0 + P.h_rows;
-      strip_warp<1, true, MIX>(a, c0, y0, y1, warp);
+      strip_warp<1, 2, MIX>(a, c0, y0, y1);
     } else if (item.type == PI_GHOST) {
       if (lane < item.count)
-        open_ghost_cell(persist_stage_args(P, d, step, item.stage), item.index + lane, 1);
+        open_ghost_cell(persist_stage_args<false>(P, d, step, item.stage), item.index + lane, 1);
     } else {
       node_bc_cell(persist_node_args(P, d, step, item.stage), item.index * 32 + lane);
     }
@@ -869,21 +834,18 @@ __global__ void __launch_bounds__(32 * PW, 8) k_batch_persistent(const __grid_co
   }
 }
 
-#undef ST
-#undef UV
-#undef NQ_
-#undef FQ
-#undef KQ
-
-// launch; with `after_node_pass`, as a programmatic dependent of the node
-// pass launched just before on `s` (it may start while the pass runs)
-inline cudaError_t launch_after_node_pass(const void* fn, unsigned blocks, unsigned threads,
-                                          size_t smem, cudaStream_t s, bool after_node_pass,
-                                          void** args) {
+// launch of one-warp CTAs; with `after_node_pass`, as a programmatic
+// dependent of the node pass launched just before on `s` (it may start while
+// the pass runs)
+inline cudaError_t launch_after_node_pass(const void* fn, unsigned blocks, cudaStream_t s,
+                                          bool after_node_pass, void** args) {
+  cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                       cudaSharedmemCarveoutMaxShared);
+  if (e != cudaSuccess) return e;
   cudaLaunchConfig_t cfg = {};
+  cfg.dynamicSmemBytes = WARP_DOUBLES * sizeof(double);
   cfg.gridDim = dim3(blocks);
-  cfg.blockDim = dim3(threads);
-  cfg.dynamicSmemBytes = smem;
+  cfg.blockDim = dim3(32);
   cfg.stream = s;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -893,78 +855,38 @@ inline cudaError_t launch_after_node_pass(const void* fn, unsigned blocks, unsig
   return cudaLaunchKernelExC(&cfg, fn, args);
 }
 
-template <int H, int WPC, int MINB, int MODE, bool MIX>
-const void* strip_fn(int kind) {
-  if (kind == K_WALL) return (const void*)k_strip<H, WPC, MINB, MODE, K_WALL, MIX>;
-  if (kind == K_OPEN) return (const void*)k_strip<H, WPC, MINB, MODE, K_OPEN, MIX>;
-  if (kind == K_WALL_OPEN) return (const void*)k_strip<H, WPC, MINB, MODE, K_WALL_OPEN, MIX>;
-  return (const void*)k_strip<H, WPC, MINB, MODE, K_PLAIN, MIX>;
+// rows per strip of shape 0..4
+constexpr int SHAPE_ROWS[5] = {8, 16, 32, 4, 2};
+template <int MODE, int UN, bool MIX>
+const void* strip_fn(bool open) {
+  return open ? (const void*)k_strip<MODE, UN, true, MIX>
+              : (const void*)k_strip<MODE, UN, false, MIX>;
+}
+const void* strip_fn(int mode, bool un, bool open, bool mixed) {
+  if (mode == 0) return mixed ? strip_fn<0, 0, true>(open) : strip_fn<0, 0, false>(open);
+  if (un) return mixed ? strip_fn<1, 1, true>(open) : strip_fn<1, 1, false>(open);
+  return mixed ? strip_fn<1, 0, true>(open) : strip_fn<1, 0, false>(open);
 }
 
-template <int H, int WPC, int MINB>
-cudaError_t launch_strip_shape(const StageArgs& a, int mode, cudaStream_t s) {
-  const size_t smem =
-      (size_t)WPC * (a.mixed ? WARP_DOUBLES_MIX : WARP_DOUBLES) * sizeof(double);
-  const bool wall = a.wall_w || a.wall_e || a.wall_s || a.wall_n;
-  const int kind = a.open ? (wall ? K_WALL_OPEN : K_OPEN) : (wall ? K_WALL : K_PLAIN);
-  const void* fn = a.mixed ? (mode == 0 ? strip_fn<H, WPC, MINB, 0, true>(kind)
-                                        : strip_fn<H, WPC, MINB, 1, true>(kind))
-                           : (mode == 0 ? strip_fn<H, WPC, MINB, 0, false>(kind)
-                                        : strip_fn<H, WPC, MINB, 1, false>(kind));
-  cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return e;
-  int sx = (a.f.nx - 2 * BC + SW - 1) / SW;
-  const int sy = (a.f.ny - 2 * BC + H * WPC - 1) / (H * WPC);
-  int ghost_ctas = a.open ? (open_ghost_count(a.f, a.open) + 32 * WPC - 1) / (32 * WPC) : 0;
-  const unsigned blocks = (unsigned)ghost_ctas + (unsigned)sx * (unsigned)sy;
-  StageArgs aa = a;
-  void* args[] = {&aa, &ghost_ctas, &sx};
-  return launch_after_node_pass(fn, blocks, 32 * WPC, smem, s, a.node_sides != 0, args);
-}
+int strips_across(const Field& f) { return (f.nx - 2 * BC + SW - 1) / SW; }
+int strips_up(const Field& f, int h) { return (f.ny - 2 * BC + h - 1) / h; }
 
-template <int H, int WPC, int MINB, bool MIX>
-const void* strip_batch_fn(int kind) {
-  return kind == BK_WALL   ? (const void*)k_strip_batch<H, WPC, MINB, K_WALL_OPEN, MIX>
-         : kind == BK_OPEN ? (const void*)k_strip_batch<H, WPC, MINB, K_OPEN, MIX>
-                           : (const void*)k_strip_batch<H, WPC, MINB, K_PLAIN, MIX>;
-}
-
-template <int H, int WPC, int MINB>
-cudaError_t launch_strip_batch_shape(BatchStageArgs& P, int kind, bool mixed, cudaStream_t s) {
-  const size_t smem = (size_t)WPC * (mixed ? WARP_DOUBLES_MIX : WARP_DOUBLES) * sizeof(double);
-  const void* fn = mixed ? strip_batch_fn<H, WPC, MINB, true>(kind)
-                         : strip_batch_fn<H, WPC, MINB, false>(kind);
-  cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return e;
-  long long ghost = 0, strips = 0;
-  for (int i = 0; i < P.ndom; i++) {
-    BatchDomain& d = P.d[i];
-    d.sx = (d.f.nx - 2 * BC + SW - 1) / SW;
-    const int sy = (d.f.ny - 2 * BC + H * WPC - 1) / (H * WPC);
-    d.ghost0 = (int)ghost;
-    d.strip0 = (int)strips;
-    if (kind == BK_OPEN || kind == BK_WALL)
-      ghost += (open_ghost_count(d.f, d.open) + 32 * WPC - 1) / (32 * WPC);
-    strips += (long long)d.sx * sy;
-  }
-  if (ghost + strips > 0x7fffffffLL) return cudaErrorInvalidValue;
-  P.ghost_ctas = (int)ghost;
-  bool pdl = false;
-  for (int i = 0; i < P.ndom; i++) pdl = pdl || P.d[i].node_sides != 0;
-  void* args[] = {&P};
-  return launch_after_node_pass(fn, (unsigned)(ghost + strips), 32 * WPC, smem, s, pdl, args);
+template <int UN, bool MIX>
+const void* strip_batch_fn(bool open) {
+  return open ? (const void*)k_strip_batch<UN, true, MIX>
+              : (const void*)k_strip_batch<UN, false, MIX>;
 }
 
 }  // namespace
 
 cudaError_t launch_batch_persistent(const PersistArgs& P, bool mixed, cudaStream_t s, int* ctas) {
-  const size_t smem = (size_t)PW * (mixed ? WARP_DOUBLES_MIX : WARP_DOUBLES) * sizeof(double);
   const void* fn = mixed ? (const void*)k_batch_persistent<true> : (const void*)k_batch_persistent<false>;
-  cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return e;
   int dev = 0, sms = 0, per_sm = 0;
-  e = cudaGetDevice(&dev);
+  cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                       cudaSharedmemCarveoutMaxShared);
+  if (e == cudaSuccess) e = cudaGetDevice(&dev);
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const size_t smem = (size_t)PW * WARP_DOUBLES * sizeof(double);
   if (e == cudaSuccess)
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, 32 * PW, smem);
   if (e != cudaSuccess) return e;
@@ -978,55 +900,54 @@ cudaError_t launch_batch_persistent(const PersistArgs& P, bool mixed, cudaStream
 cudaError_t launch_strip_batch(BatchStageArgs& P, int kind, int shape, bool mixed,
                                cudaStream_t s) {
   if (P.ndom <= 0) return cudaSuccess;
-  if (P.ndom > BATCH_MAX) return cudaErrorInvalidValue;
-  switch (shape) {
-    case 0: return launch_strip_batch_shape<8, 4, 4>(P, kind, mixed, s);
-    case 1: return launch_strip_batch_shape<16, 4, 4>(P, kind, mixed, s);
-    case 2: return launch_strip_batch_shape<16, 4, 5>(P, kind, mixed, s);
-    case 3: return launch_strip_batch_shape<16, 2, 8>(P, kind, mixed, s);
-    case 4: return launch_strip_batch_shape<16, 8, 2>(P, kind, mixed, s);
+  if (P.ndom > BATCH_MAX || shape < 0 || shape > 4) return cudaErrorInvalidValue;
+  int h = SHAPE_ROWS[shape];
+  const bool open = kind == BK_OPEN || kind == BK_WALL;
+  long long ghost = 0, strips = 0;
+  bool pdl = false;
+  for (int i = 0; i < P.ndom; i++) {
+    BatchDomain& d = P.d[i];
+    d.sx = strips_across(d.f);
+    d.ghost0 = (int)ghost;
+    d.strip0 = (int)strips;
+    if (open) ghost += (open_ghost_count(d.f, d.open) + 31) / 32;
+    strips += (long long)d.sx * strips_up(d.f, h);
+    pdl = pdl || d.node_sides != 0;
   }
-  return cudaErrorInvalidValue;
-}
-
-template <int H, int WPC, int MINB>
-cudaError_t launch_strip_masked_shape(const StageArgs& a, cudaStream_t s) {
-  const size_t smem = (size_t)WPC * WARP_DOUBLES * sizeof(double);
-  const void* fn = (const void*)k_strip<H, WPC, MINB, 2, K_PLAIN, false>;
-  cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return e;
-  int sx = (a.box_x1 - (a.box_x0 & ~1) + SW) / SW;
-  const int sy = (a.box_y1 - a.box_y0 + H * WPC) / (H * WPC);
-  int ghost_ctas = 0;
-  StageArgs aa = a;
-  void* args[] = {&aa, &ghost_ctas, &sx};
-  return launch_after_node_pass(fn, (unsigned)sx * (unsigned)sy, 32 * WPC, smem, s, false, args);
+  if (ghost + strips > 0x7fffffffLL) return cudaErrorInvalidValue;
+  P.ghost_ctas = (int)ghost;
+  const void* fn = P.stage != 1 ? (mixed ? strip_batch_fn<1, true>(open) : strip_batch_fn<1, false>(open))
+                                : (mixed ? strip_batch_fn<0, true>(open) : strip_batch_fn<0, false>(open));
+  void* args[] = {&P, &h};
+  return launch_after_node_pass(fn, (unsigned)(ghost + strips), s, pdl, args);
 }
 
 // L(u) of a buffer-layer grid at its interior_pt points (MODE 2) over the
-// border box [box_x0, box_x1] x [box_y0, box_y1] (box_x0, box_y0 >= BC:
-// every copied row and column lies inside the grid).  Strips of 16 rows (2
-// warps per CTA, 8 CTAs per SM) where they fill the GPU's 148 x 16 warp
-// slots, else of 8 rows (4 warps per CTA) for twice the warps: layers are
-// often thin bands.  Needs strip_layout_ok(a).
+// border box [box_x0, box_x1] x [box_y0, box_y1] (box_x0, box_y0 >= BC, so
+// every row and column read lies inside the grid).  Strips of 16 rows where
+// they fill the GPU's 148 x 16 warp slots, else of 8 rows for twice the
+// warps: layers are often thin bands.
 cudaError_t launch_strip_masked(const StageArgs& a, cudaStream_t s) {
-  const long long sx = (a.box_x1 - (a.box_x0 & ~1) + SW) / SW;
-  const long long warps16 = sx * ((a.box_y1 - a.box_y0 + 16) / 16);
-  if (warps16 >= 148LL * 16) return launch_strip_masked_shape<16, 2, 8>(a, s);
-  return launch_strip_masked_shape<8, 4, 4>(a, s);
+  int sx = (a.box_x1 - (a.box_x0 & ~1) + SW) / SW;
+  const int rows = a.box_y1 - a.box_y0 + 1;
+  int h = (long long)sx * ((rows + 15) / 16) >= 148LL * WARPS ? 16 : 8;
+  int ghost_ctas = 0;
+  StageArgs aa = a;
+  void* args[] = {&aa, &ghost_ctas, &sx, &h};
+  return launch_after_node_pass(strip_fn<2, 0, false>(false), (unsigned)sx * (unsigned)((rows + h - 1) / h), s,
+                                false, args);
 }
 
-// shape id -> (rows per warp, warps per CTA, minimum resident CTAs per SM
-// requested from the register allocator)
 cudaError_t launch_strip_stage(const StageArgs& a, int mode, int shape, cudaStream_t s) {
-  switch (shape) {
-    case 0: return launch_strip_shape<8, 4, 4>(a, mode, s);
-    case 1: return launch_strip_shape<16, 4, 4>(a, mode, s);
-    case 2: return launch_strip_shape<16, 4, 5>(a, mode, s);
-    case 3: return launch_strip_shape<16, 2, 8>(a, mode, s);
-    case 4: return launch_strip_shape<16, 8, 2>(a, mode, s);
-  }
-  return cudaErrorInvalidValue;
+  if (shape < 0 || shape > 4) return cudaErrorInvalidValue;
+  int h = SHAPE_ROWS[shape], sx = strips_across(a.f);
+  int ghost_ctas = a.open ? (open_ghost_count(a.f, a.open) + 31) / 32 : 0;
+  const bool open = a.open != 0;
+  const void* fn = strip_fn(mode, a.stage != 1, open, a.mixed);
+  StageArgs aa = a;
+  void* args[] = {&aa, &ghost_ctas, &sx, &h};
+  return launch_after_node_pass(fn, (unsigned)ghost_ctas + (unsigned)sx * (unsigned)strips_up(a.f, h),
+                                s, a.node_sides != 0, args);
 }
 
 }  // namespace dim2d
