@@ -44,6 +44,17 @@ enum OpenSection : int {
   OPEN_ALL = 255
 };
 
+// Ghost runs of the strip launches: a warp integrates up to OPEN_RUN cells of
+// one ghost layer along an open edge, one more the corner cells.
+constexpr int OPEN_RUN = 28;
+inline int open_run_count(const Field& f, int mask) {
+  int n = mask >> 4 ? 1 : 0;
+  for (int side = 0; side < 4; side++)
+    if (mask >> side & 1)
+      n += BC * (((side < 2 ? f.nx : f.ny) - 2 * BC + OPEN_RUN - 1) / OPEN_RUN);
+  return n;
+}
+
 // Coefficients of the strip kernel's node quantities and face fluxes
 // (dim2d_strip.cu), from the physical constants and the grid step: computed
 // on the host once per launch so that the kernel reads them as constants.
@@ -313,9 +324,10 @@ struct PItem {
   int dom;
   int type;   // PItemType
   int stage;  // 1, 2, 3
-  int index;  // strip: band * sx + column strip; ghost: first cell (open_ghost_cell
-              // numbering); node: 32-cell group of node_bc_cell
-  int count;  // ghost: cells of the item (<= 32)
+  int index;  // strip: band * sx + column strip; ghost: side << 24 | layer << 20 | first
+              // cell along the edge (side 4: corner cells); node: 32-cell group of node_bc_cell
+  int count;  // ghost: cells of the run (<= OPEN_RUN), or OPEN_* mask of the corners;
+              // strip: 1 if it reads a ghost cell of the node pass
   int band;   // row band (strip, ghost)
 };
 

@@ -37,7 +37,6 @@
 
 #include "dim2d_internal.h"
 #include "dim2d_nodebc.cuh"
-#include "dim2d_open.cuh"
 
 using namespace dim2d;
 
@@ -55,37 +54,33 @@ NodeBcArgs node_args_of(const dim2d_handle* h) {
 }
 
 // Ghost-cell items of one field's open sections, by row band: runs of at
-// most 32 cells of open_ghost_cell's numbering (sections S, N, W, E, SW,
-// SE, NW, NE in that order, skipping the closed ones), each inside one band:
-// the S edge and S corners in band 0, the N edge and N corners in the last
-// band, the W and E edge cells of the rows of each band in that band.
+// most OPEN_RUN cells of one layer along an edge, each inside one band: the S
+// edge and S corners in band 0, the N edge and N corners in the last band,
+// the W and E edge cells of the rows of each band in that band.
 struct GhostRun {
-  int first, count, band;
+  int index, count, band;
 };
 std::vector<GhostRun> ghost_runs(const dim2d_handle* h, int rows, int nb) {
   std::vector<GhostRun> out;
   const int mask = h->open_mask;
   if (!mask) return out;
   const int ey = h->f.ny - 2 * BC;
-  auto add = [&](int first, int n, int band) {
-    for (int o = 0; o < n; o += 32) out.push_back(GhostRun{first + o, std::min(32, n - o), band});
+  auto add = [&](int side, int first, int n, int band) {
+    for (int layer = 0; layer < BC; layer++)
+      for (int o = 0; o < n; o += OPEN_RUN)
+        out.push_back(GhostRun{side << 24 | layer << 20 | (BC + first + o),
+                               std::min(OPEN_RUN, n - o), band});
   };
-  int off = 0;
-  for (int sec = 0; sec < 8; sec++) {
-    if (!(mask >> sec & 1)) continue;
-    const int cells = open_section_cells(h->f, sec);
-    if (sec == 0 || sec == 4 || sec == 5) {
-      add(off, cells, 0);
-    } else if (sec == 1 || sec == 6 || sec == 7) {
-      add(off, cells, nb - 1);
-    } else {  // W or E edge: BC columns of ey cells each
-      for (int b = 0; b < nb; b++) {
-        const int r0 = b * rows, n = b == nb - 1 ? ey - r0 : rows;
-        for (int col = 0; col < BC; col++) add(off + col * ey + r0, n, b);
-      }
-    }
-    off += cells;
-  }
+  for (int side = 0; side < 2; side++)
+    if (mask >> side & 1) add(side, 0, h->f.nx - 2 * BC, side ? nb - 1 : 0);
+  for (int side = 2; side < 4; side++)
+    if (mask >> side & 1)
+      for (int b = 0; b < nb; b++)
+        add(side, b * rows, b == nb - 1 ? ey - b * rows : rows, b);
+  if (mask & (OPEN_SW | OPEN_SE))
+    out.push_back(GhostRun{4 << 24, mask & (OPEN_SW | OPEN_SE), 0});
+  if (mask & (OPEN_NW | OPEN_NE))
+    out.push_back(GhostRun{4 << 24, mask & (OPEN_NW | OPEN_NE), nb - 1});
   return out;
 }
 
@@ -192,7 +187,7 @@ int persist_build(PersistPlan& pl, const std::vector<dim2d_handle*>& hs,
       for (int j : by_size) {
         if (band >= dom[j].nb) continue;
         for (const GhostRun& g : ghosts[j])
-          if (g.band == band) items.push_back(PItem{j, PI_GHOST, st, g.first, g.count, band});
+          if (g.band == band) items.push_back(PItem{j, PI_GHOST, st, g.index, g.count, band});
         for (int q = 0; q < dom[j].sx; q++)
           items.push_back(PItem{j, PI_STRIP, st, band * dom[j].sx + q,
                                 strip_reads_node_ghosts(hs[j], dom[j], band, q, rows), band});

@@ -37,14 +37,13 @@
 // 96 registers (92; spills), three or four rows per pass (as fast, larger).
 //
 // On a field with open sections the launch also integrates their ghost
-// cells (open_ghost_cell, one thread each): they take the first CTAs of the
-// grid, so their long dependent chains start first and overlap the strips.
-// Ghost and interior cells read the same input and write disjoint cells.
+// cells (open_run, one warp per run): they take the first CTAs of the grid, so
+// that they overlap the strips.  Ghost and interior cells read the same input
+// and write disjoint cells.
 // the ghost-cell and node-pass code of this file runs inside the persistent
 // kernel, whose inputs change during the launch: coherent loads
 #define DIM2D_COHERENT_LOADS
 #include "dim2d_nodebc.cuh"
-#include "dim2d_open.cuh"
 
 namespace dim2d {
 
@@ -181,21 +180,22 @@ __device__ __forceinline__ NodeUV node_uv(double r, double mx, double my) {
   n.v = mul(my, n.ir);
   return n;
 }
-// the rest; dw, de, ds, dn = density differences to the west (r - r_w), east
-// (r_e - r), south and north node
+// the rest; dw = density difference to the west node, d1x, d1y = sums and
+// d2x, d2y = differences of the density differences to both sides (the
+// undivided centred first and second differences)
 template <typename T>
 __device__ __forceinline__ NodeQ<T> node(const NodeUV& n, double r, double mx, double my,
-                                         double e, double dw, double de, double ds, double dn,
-                                         const StripCoef<double>& c) {
+                                         double e, double dw, double d1x, double d2x, double d1y,
+                                         double d2y, const StripCoef<double>& c) {
   const double cp = mul(c.c15cv * r, n.inv);
   const double m3r2 = mul(-3.0 * r, r);
   // W = E - rho|u|^2/2 + 3 rho^2
   const double w = fma(-0.5, fma(mx, n.u, my * n.v), e) - m3r2;
   const double p = fma(cp, w + w, m3r2);
-  const double gx = mul(c.gx, de + dw), gy = mul(c.gy, dn + ds);
+  const double gx = mul(c.gx, d1x), gy = mul(c.gy, d1y);
   NodeQ<T> q;
   q.th = mul(n.ir, fma(-2.0, fma(gx, gx, gy * gy), w));
-  q.lap = (T)fma(c.lx, de - dw, c.ly * (dn - ds));
+  q.lap = (T)fma(c.lx, d2x, c.ly * d2y);
   q.r = (T)r;
   q.mx = (T)mx;
   q.my = (T)my;
@@ -211,6 +211,13 @@ __device__ __forceinline__ NodeQ<T> node(const NodeUV& n, double r, double mx, d
   q.gy = (T)gy;
   q.dw = (T)dw;
   return q;
+}
+
+template <typename T>  // dw, de, ds, dn = density differences to the four nodes around
+__device__ __forceinline__ NodeQ<T> node(const NodeUV& n, double r, double mx, double my,
+                                         double e, double dw, double de, double ds, double dn,
+                                         const StripCoef<double>& c) {
+  return node<T>(n, r, mx, my, e, dw, de + dw, de - dw, dn + ds, dn - ds, c);
 }
 
 // the face pass's type and coefficients
@@ -283,8 +290,8 @@ __device__ __forceinline__ void wall_face2(const FaceSums<T>& f, const FaceCoef<
 // quantities of row y, ul, vl = the left column's velocity, gyu, gyv =
 // undivided velocity differences across row y
 template <typename T>
-__device__ __forceinline__ void x_face(const NodeQ<T>& n, T ul, T vl, T gyu, T gyv,
-                                       const StripCoef<T>& c, double cth, T F[3], double* F3) {
+__device__ __forceinline__ FaceSums<T> x_sums(const NodeQ<T>& n, T ul, T vl, T gyu, T gyv,
+                                              double cth) {
   FaceSums<T> f;
   const T cl = from_left(n.cp);
   f.smn = from_left(n.mx) + n.mx;
@@ -307,7 +314,7 @@ __device__ __forceinline__ void x_face(const NodeQ<T>& n, T ul, T vl, T gyu, T g
   f.dunt = from_left(gyu) + gyu;
   f.dutt = from_left(gyv) + gyv;
   f.lap = from_left(n.lap) + n.lap;
-  face2(f, c.x, c.s, F, F3);
+  return f;
 }
 
 // y-face between rows y (b) and y+1 (t) of the lane's column: dr = density
@@ -333,6 +340,234 @@ __device__ __forceinline__ FaceSums<T> y_sums(const NodeQ<T>& b, const NodeQ<T>&
   f.dutt = gxub + gxut;
   f.lap = b.lap + t.lap;
   return f;
+}
+
+// ---- open (Hedstrom) ghost cells ----------------------------------------
+// What open_ghost_cell (dim2d_open.cuh) evaluates one cell per thread -- both
+// faces of a cell from scratch, some 20 node primitives and a dependent chain
+// of divisions and square roots that took 12 us whatever the field's size --
+// done by a warp for a run of one layer's cells along an edge: a lane holds
+// one position along the edge and the three nodes across it (both ghost
+// layers and the first interior one), and neighbours come by shuffle as in the
+// strips.  Per RK3 step: 64^2 open 30.7 -> 12.3 us, 301x187 half_wall_S_open
+// 59 -> 29 us, 1024^2 open 82 -> 69 us.  Both layers in one warp would halve
+// the loads but need more registers than the strips leave (160 bytes of spill
+// in the batched kernels).
+
+// Characteristic time derivative (hedstrom_xy_module.f:445-558 with the
+// node's own eigenquantities) in the edge's frame: u along the edge, v across
+// it, g.. = one-sided derivatives across it; out = (mass, momentum along,
+// momentum across, energy).  The speed of sound of sound_speed() with its
+// radicands multiplied out: c^2 = 3 (e + (P + 3 rho^2)/cv_r)/(rho (3 - rho)),
+// e = P + rho^2 (2 rho - 3); where one of those radicands is negative the
+// value is NaN there, and here.
+__device__ __forceinline__ void char_term_run(double r, const NodeUV& n, double p, double gr,
+                                              double gu, double gv, double gp, bool right,
+                                              const DimConst& k, double out[4]) {
+  const double u = n.u, v = n.v;
+  const double ee = fma(r * r, fma(2.0, r, -3.0), p), pe = fma(3.0 * r, r, p);
+  double c2 = fma(3.0, ee, k.c3cv * pe) * n.inv;
+  if (!(r >= 0.0 && (3.0 - r) * ee >= 0.0 && pe * ee >= 0.0)) c2 = NAN;
+  const double c = sqrt(c2), ic2 = 1.0 / c2;
+  const double qc = 0.5 * r * c;
+  auto amp = [&](double ev, double lg) {
+    return (right ? ev <= 0.0 : ev >= 0.0) ? 0.0 : -ev * lg;  // openbc_operators_module.f:97-136
+  };
+  const double a0 = amp(v, gu), a1 = amp(v, fma(-ic2, gp, gr));
+  const double a2 = amp(v - c, fma(-qc, gv, 0.5 * gp)), a3 = amp(v + c, fma(qc, gv, 0.5 * gp));
+  const double tp = a2 + a3, tr = fma(ic2, tp, a1), tv = n.ir * c * ic2 * (a3 - a2);
+  // conservative <- primitive Jacobian, ns_vdw2d_prim_module.f:249-320
+  const double de = 0.5 * fma(u, u, v * v) - 6.0 * r -
+                    1.0 / 3.0 * k.cv_r * fma(9.0 * (r - 2.0), r, p);
+  out[0] = tr;
+  out[1] = fma(tr, u, a0 * r);
+  out[2] = fma(tr, v, tv * r);
+  out[3] = fma(tr, de, r * fma(a0, u, tv * v)) + tp * (k.cv_r * (1.0 - r / 3.0));
+}
+
+__device__ __forceinline__ double pressure(const NodeUV& n, double r, double mx, double my,
+                                           double e, const DimConst& k) {
+  const double m3r2 = mul(-3.0 * r, r);
+  const double w = fma(-0.5, fma(mx, n.u, my * n.v), e) - m3r2;
+  return fma(mul(k.c15cv * r, n.inv), w + w, m3r2);
+}
+
+// L(u) (MODE 0) or stage update (MODE 1) of one ghost cell at offset o
+template <int MODE>
+__device__ __forceinline__ void store_ghost(const StageArgs& a, size_t o, const double q[4],
+                                            double L[4], const double un[4]) {
+  if (a.k.gravity_ac) {  // openbc_operators_module.f:354-372
+    L[2] = fma(-q[0], a.k.gravity, L[2]);
+    L[3] = fma(-q[2], a.k.gravity, L[3]);
+  }
+#pragma unroll
+  for (int v = 0; v < 4; v++) {
+    double out = L[v];
+    if (MODE == 1) {
+      out = fma(a.dt, L[v], q[v]);
+      if (a.stage != 1) out = fma(a.b, un[v], (1.0 - a.b) * out);
+    }
+    a.uout[o + v * a.f.plane] = out;
+  }
+}
+
+// One ghost layer (0 inner, 1 outer) of `count` <= OPEN_RUN cells from position
+// `first` along edge `side` (0..3 = S, N, W, E).  Lane l holds position first-2+l; cells are
+// lanes 2 .. count+1, faces lanes 2 .. count+2.  Inner layer: the interior
+// operators across the edge; outer layer: the one-sided ones (the *_L0 / *_R0
+// sets, bc_operators_openbc_normal_class.f:563-713), whose second derivative
+// across the edge is the inner layer's.
+template <int MODE>
+__device__ __forceinline__ void open_edge_run(const StageArgs& a, int side, int layer, int first,
+                                              int count) {
+  const int lane = threadIdx.x & 31;
+  const Field& f = a.f;
+  const DimConst& k = a.k;
+  const bool ye = side >= 2, hi = side & 1;  // edge along y; N or E
+  const size_t along = ye ? f.pitch : 1, across = ye ? 1 : f.pitch;
+  const int na = ye ? f.ny : f.nx, nc = ye ? f.nx : f.ny;
+  const int c0 = hi ? nc - 3 : 0;  // the three nodes across: c0, c0+1, c0+2
+  const size_t o0 = min(max(first - 2 + lane, 0), na - 1) * along + c0 * across;
+  const size_t V = f.plane, vs = ye ? 2 * V : V, vc = ye ? V : 2 * V;
+  double r[3], ms[3], mc[3], e[3], un[4];
+#pragma unroll
+  for (int j = 0; j < 3; j++) {
+    const double* p = a.uin + o0 + j * across;
+    r[j] = __ldcg(p);
+    ms[j] = __ldcg(p + vs);
+    mc[j] = __ldcg(p + vc);
+    e[j] = __ldcg(p + 3 * V);
+  }
+  const bool outer = layer == 1;
+  const int jl = outer ? (hi ? 2 : 0) : 1;  // the layer's node
+  const size_t o = o0 + jl * across;
+#pragma unroll
+  for (int v = 0; v < 4; v++)
+    un[v] = MODE == 1 && a.stage != 1 ? __ldcg(a.u0 + o + v * V) : 0.0;
+
+  // coefficients in the edge's frame (x = along it, y = across it)
+  const FaceCoef<double>& ca = ye ? a.c.y : a.c.x;
+  StripCoef<double> c;
+  c.c15cv = a.c.c15cv;
+  c.gx = ye ? a.c.gy : a.c.gx;
+  c.gy = ye ? a.c.gx : a.c.gy;
+  c.lx = ye ? a.c.ly : a.c.lx;
+  c.ly = ye ? a.c.lx : a.c.ly;
+  const double rda = ye ? a.rdy : a.rdx, rdc = ye ? a.rdx : a.rdy;
+
+  NodeUV n[3];
+  double p[3];
+#pragma unroll
+  for (int j = 0; j < 3; j++) {
+    n[j] = node_uv(r[j], ms[j], mc[j]);
+    p[j] = pressure(n[j], r[j], ms[j], mc[j], e[j], k);
+  }
+  auto own = [&](const double* q) { return outer ? (hi ? q[2] : q[0]) : q[1]; };
+  // difference across the edge that the layer's one-sided operators take, and
+  // twice the undivided derivative of its tangential operators
+  auto side_diff = [&](double q0, double q1, double q2) { return hi == outer ? q2 - q1 : q1 - q0; };
+  auto twice = [&](double q0, double q1, double q2) {
+    return outer ? 2.0 * (hi ? q2 - q1 : q1 - q0) : (q2 - q1) + (q1 - q0);
+  };
+  const double rl = own(r), msl = own(ms), mcl = own(mc), el = own(e), pl = own(p);
+  const NodeUV nl = outer ? (hi ? n[2] : n[0]) : n[1];
+  const double dw = rl - from_left(rl), de = from_right(rl) - rl;
+  const NodeQ<double> q =
+      node<double>(nl, rl, msl, mcl, el, dw, de + dw, de - dw, twice(r[0], r[1], r[2]),
+                   (r[2] - r[1]) - (r[1] - r[0]), c);
+  const FaceSums<double> fs =
+      x_sums(q, from_left(q.u), from_left(q.v), twice(n[0].u, n[1].u, n[2].u),
+             twice(n[0].v, n[1].v, n[2].v), ca.th);
+  double F[3], F3;
+  face2(fs, ca, a.c.s, F, &F3);
+  if (ye && a.wall_s && first == BC) {
+    // the face under the first interior row carries the wall corner's flux
+    // (bc_operators_wall_xy_class.f:702-854)
+    double W[3], W3;
+    wall_face2(fs, ca, q.th, a.dy, wall_heat_flux(a.wall, a.xmap0 + (c0 + jl) * a.dx), k, W, &W3);
+    if (lane == 2) {
+      F[0] = W[0];
+      F[1] = W[1];
+      F[2] = W[2];
+      F3 = W3;
+    }
+  }
+  double D[4];
+#pragma unroll
+  for (int v = 0; v < 3; v++) D[v] = F[v] - from_right(F[v]);
+  D[3] = F3 - from_right(F3);
+  double ch[4];
+  char_term_run(rl, nl, pl, rdc * side_diff(r[0], r[1], r[2]),
+                rdc * side_diff(n[0].u, n[1].u, n[2].u),
+                rdc * side_diff(n[0].v, n[1].v, n[2].v), rdc * side_diff(p[0], p[1], p[2]), hi, k,
+                ch);
+  if (lane >= 2 && lane < 2 + count) {
+    const double h = 0.5 * rda;
+    const double qc[4] = {rl, ye ? mcl : msl, ye ? msl : mcl, el};
+    double L[4] = {fma(h, D[0], ch[0]), ye ? fma(h, D[2], ch[2]) : fma(h, D[1], ch[1]),
+                   ye ? fma(h, D[1], ch[1]) : fma(h, D[2], ch[2]), fma(h, D[3], ch[3])};
+    store_ghost<MODE>(a, o, qc, L, un);
+  }
+}
+
+// The corner cells of the sections in `mask`, lanes 0..15 (four per corner,
+// SW, SE, NW, NE): characteristic terms of both directions.
+template <int MODE>
+__device__ __forceinline__ void open_corner_cells(const StageArgs& a, int mask) {
+  const int lane = threadIdx.x & 31, c = lane >> 2;
+  if (lane >= 16 || !(mask >> (4 + c) & 1)) return;
+  const Field& f = a.f;
+  const DimConst& k = a.k;
+  const bool east = c & 1, north = c >> 1;
+  const int x = (east ? f.nx - BC : 0) + (lane & 1), y = (north ? f.ny - BC : 0) + (lane >> 1 & 1);
+  const size_t o = (size_t)y * f.pitch + x, V = f.plane;
+  // the node and its neighbours inwards along x and along y
+  const ptrdiff_t d[3] = {0, east ? -1 : 1, north ? -(ptrdiff_t)f.pitch : f.pitch};
+  double q[3][4], un[4];
+#pragma unroll
+  for (int j = 0; j < 3; j++)
+#pragma unroll
+    for (int v = 0; v < 4; v++) q[j][v] = __ldcg(a.uin + o + d[j] + v * V);
+#pragma unroll
+  for (int v = 0; v < 4; v++)
+    un[v] = MODE == 1 && a.stage != 1 ? __ldcg(a.u0 + o + v * V) : 0.0;
+  NodeUV n[3];
+  double p[3];
+#pragma unroll
+  for (int j = 0; j < 3; j++) {
+    n[j] = node_uv(q[j][0], q[j][1], q[j][2]);
+    p[j] = pressure(n[j], q[j][0], q[j][1], q[j][2], q[j][3], k);
+  }
+  const double sx = east ? a.rdx : -a.rdx, sy = north ? a.rdy : -a.rdy;
+  const NodeUV t{n[0].inv, n[0].ir, n[0].v, n[0].u};  // along y, across x
+  double cx[4], cy[4], L[4];
+  char_term_run(q[0][0], t, p[0], sx * (q[0][0] - q[1][0]), sx * (n[0].v - n[1].v),
+                sx * (n[0].u - n[1].u), sx * (p[0] - p[1]), east, k, cx);
+  char_term_run(q[0][0], n[0], p[0], sy * (q[0][0] - q[2][0]), sy * (n[0].u - n[2].u),
+                sy * (n[0].v - n[2].v), sy * (p[0] - p[2]), north, k, cy);
+  L[0] = cx[0] + cy[0];
+  L[1] = cx[2] + cy[1];
+  L[2] = cx[1] + cy[2];
+  L[3] = cx[3] + cy[3];
+  store_ghost<MODE>(a, o, q[0], L, un);
+}
+
+// ghost run number m of a launch: the runs of the open edges S, N, W, E, then
+// one for the corners
+template <int MODE>
+__device__ __forceinline__ void open_run(const StageArgs& a, int m) {
+  for (int side = 0; side < 4; side++) {
+    if (!(a.open >> side & 1)) continue;
+    const int cells = (side < 2 ? a.f.nx : a.f.ny) - 2 * BC;
+    const int runs = BC * ((cells + OPEN_RUN - 1) / OPEN_RUN);
+    if (m < runs) {
+      const int at = m / BC * OPEN_RUN;
+      open_edge_run<MODE>(a, side, m % BC, BC + at, min(OPEN_RUN, cells - at));
+      return;
+    }
+    m -= runs;
+  }
+  open_corner_cells<MODE>(a, a.open);
 }
 
 // The strip of one warp: columns c0 .. c0+29 (interior ones), rows y0 ..
@@ -456,7 +691,7 @@ __device__ __forceinline__ void strip_warp(const StageArgs& a, int c0, int y0, i
     // x-face of row y, and the right one from lane+1
     T Fx[3];
     double fx3;
-    x_face(n0, ul0, vl0, gyu, gyv, c, cd.x.th, Fx, &fx3);
+    face2(x_sums(n0, ul0, vl0, gyu, gyv, cd.x.th), c.x, c.s, Fx, &fx3);
     double D[4];  // 2 (F_left - F_right)
 #pragma unroll
     for (int v = 0; v < 3; v++) D[v] = (double)Fx[v] - (double)from_right(Fx[v]);
@@ -558,7 +793,7 @@ __global__ void __launch_bounds__(32, WARPS) k_strip(const __grid_constant__ Sta
   if (OPEN) {
     if (b < ghost_ctas) {
       if (a.node_sides) wait_for_node_pass();  // ghost frames reach the wall rows
-      open_ghost_cell(a, b * 32 + threadIdx.x, MODE);
+      open_run<MODE>(a, b);
       return;
     }
     b -= ghost_ctas;
@@ -624,7 +859,7 @@ __global__ void __launch_bounds__(32, WARPS)
       const int i = batch_domain<true>(P, b);
       const StageArgs a = batch_stage_args<false>(P, i);
       if (a.node_sides) wait_for_node_pass();
-      open_ghost_cell(a, (b - P.d[i].ghost0) * 32 + threadIdx.x, 1);
+      open_run<1>(a, b - P.d[i].ghost0);
       return;
     }
     b -= P.ghost_ctas;
@@ -813,8 +1048,11 @@ __global__ void __launch_bounds__(32 * PW, 8) k_batch_persistent(const __grid_co
       const int y1 = item.band == d.nb - 1 ? d.f.ny - BC : y0 + P.h_rows;
       strip_warp<1, 2, MIX>(a, c0, y0, y1);
     } else if (item.type == PI_GHOST) {
-      if (lane < item.count)
-        open_ghost_cell(persist_stage_args<false>(P, d, step, item.stage), item.index + lane, 1);
+      const StageArgs a = persist_stage_args<false>(P, d, step, item.stage);
+      const int side = item.index >> 24;
+      if (side < 4)
+        open_edge_run<1>(a, side, item.index >> 20 & 1, item.index & 0xfffff, item.count);
+      else open_corner_cells<1>(a, item.count);
     } else {
       node_bc_cell(persist_node_args(P, d, step, item.stage), item.index * 32 + lane);
     }
@@ -910,7 +1148,7 @@ cudaError_t launch_strip_batch(BatchStageArgs& P, int kind, int shape, bool mixe
     d.sx = strips_across(d.f);
     d.ghost0 = (int)ghost;
     d.strip0 = (int)strips;
-    if (open) ghost += (open_ghost_count(d.f, d.open) + 31) / 32;
+    if (open) ghost += open_run_count(d.f, d.open);
     strips += (long long)d.sx * strips_up(d.f, h);
     pdl = pdl || d.node_sides != 0;
   }
@@ -941,7 +1179,7 @@ cudaError_t launch_strip_masked(const StageArgs& a, cudaStream_t s) {
 cudaError_t launch_strip_stage(const StageArgs& a, int mode, int shape, cudaStream_t s) {
   if (shape < 0 || shape > 4) return cudaErrorInvalidValue;
   int h = SHAPE_ROWS[shape], sx = strips_across(a.f);
-  int ghost_ctas = a.open ? (open_ghost_count(a.f, a.open) + 31) / 32 : 0;
+  int ghost_ctas = open_run_count(a.f, a.open);
   const bool open = a.open != 0;
   const void* fn = strip_fn(mode, a.stage != 1, open, a.mixed);
   StageArgs aa = a;

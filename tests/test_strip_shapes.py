@@ -1,0 +1,67 @@
+"""The strip kernels at the sizes where their tiling changes: one warp's 30
+columns and its neighbours' halo, the strip heights of the five shapes and
+their remainders, and the 28-cell runs in which the ghost layers of open
+edges are integrated -- against the oracle, over all cells that have a time
+derivative (bars: 1e-12 normwise for the time derivative, as in the parity
+tests; 1e-12 after two steps, whose rounding is dt times that)."""
+import numpy as np
+import pytest
+
+from dim2d_finite_volume_b200 import workloads
+
+pytestmark = pytest.mark.gpu
+
+# interior sizes: the smallest field, one column or row short of, at and past
+# a run (28), a strip (30), two of them, and a strip height (16, 32)
+SIZES = [(4, 4), (27, 5), (28, 16), (29, 17), (30, 31), (31, 33), (56, 2 * 28), (57, 15), (61, 32)]
+
+
+@pytest.fixture(scope="module")
+def F():
+    from dim2d_finite_volume_b200 import field
+    return field
+
+
+@pytest.mark.parametrize("preset", ["periodic_xy", "hedstrom_xy", "wall_S_open",
+                                    "half_wall_S_open"])
+@pytest.mark.parametrize("n,ny", SIZES)
+def test_tiling_edges(oracle, F, preset, n, ny):
+    d = workloads.domain(n, ny, T0=0.95, bubbles=[(0.0, -0.3, 0.2)], mach=0.05, bc=preset, li=0.2)
+    rng = np.random.default_rng(n * 100 + ny)
+    q = d["nodes"]
+    q[1:3] += 0.02 * rng.standard_normal(q[1:3].shape)
+    if preset == "periodic_xy":
+        workloads.fill_periodic_ghosts(q)
+        cfg = oracle.make_cfg(d["nx"], d["ny"], periodic=True)
+    else:
+        ch, ty, od = F._preset(preset)
+        cfg = oracle.make_cfg(d["nx"], d["ny"], bc_choice=ch, bc_type=ty, bc_order=od)
+        if preset != "hedstrom_xy":
+            oracle.apply_bc_on_nodes(cfg, 0.0, d["x_map"], d["y_map"], q.copy(), q)
+    td = oracle.compute_time_dev(cfg, 0.0, q, d["x_map"], d["y_map"])
+    has = np.abs(td) < 1e30  # cells without a time derivative hold debug_real
+    ref = q.copy()
+    try:
+        oracle.integrate(cfg, ref, d["x_map"], d["y_map"], 0.0, d["dt"], 2)
+    except RuntimeError:
+        # no wall root for this state, where the reference stops: its time
+        # derivative is compared, no step
+        assert "wall" in preset
+        oracle.lib().orc_clear_status()
+        ref = None
+    # the wall operator leaves parts of its two ghost rows untouched
+    rows = slice(2 if "wall" in preset else 0, None)
+    for variant in (1, 2, 4, 5):
+        with F.Field(d["nx"], d["ny"], bc=preset) as fld:
+            fld.ini(q, d["x_map"], d["y_map"])
+            fld.variant = variant
+            got_td = fld.compute_time_dev()
+            if ref is not None:
+                fld.integrate(d["dt"], 2)
+                got = fld.download()
+        for v in range(4):
+            m = has[v]
+            assert np.abs(got_td[v] - td[v])[m].max() <= 1e-12 * np.abs(td[v][m]).max(), (variant, v)
+            if ref is not None:
+                a, b = got[v][rows], ref[v][rows]
+                assert np.abs(a - b).max() <= 1e-12 * np.abs(b).max(), (variant, v)
