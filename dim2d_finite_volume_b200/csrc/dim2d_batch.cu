@@ -56,7 +56,7 @@ struct dim2d_batch {
   std::vector<dim2d_handle*> m;
   std::vector<double> dt;
   dim2d_params p{};
-  int shape[NGROUPS] = {1, 1, 1, 1, 1, 1, 1, 1};
+  int shape[NGROUPS];  // strip shape of each group, SHAPE_BY_SIZE until set or tuned
   bool use_graphs = true;
   cudaGraphExec_t graph[2] = {nullptr, nullptr};
   long long graph_launches[2] = {0, 0};
@@ -305,6 +305,7 @@ int dim2d_batch_create(dim2d_batch** out) {
   if (!out) return set_error(DIM2D_ERR_ARG, "batch_create: null argument");
   *out = nullptr;
   dim2d_batch* b = new dim2d_batch();
+  std::fill(b->shape, b->shape + NGROUPS, SHAPE_BY_SIZE);
   cudaGetDevice(&b->device);
   cudaError_t e = cudaStreamCreateWithFlags(&b->own_stream, cudaStreamNonBlocking);
   for (int g = 0; g < NGROUPS && e == cudaSuccess; g++) {
@@ -561,7 +562,8 @@ int dim2d_batch_autotune(dim2d_batch* b, int chosen[8], double* times_ms) {
       b->shape[g] = best_shape;
       drop_batch_graphs(b);
     }
-    if (chosen) chosen[g] = b->shape[g];
+    // a group that was neither set nor tuned (empty) reports shape 1
+    if (chosen) chosen[g] = b->shape[g] == SHAPE_BY_SIZE ? 1 : b->shape[g];
   }
   if (e0) cudaEventDestroy(e0);
   if (e1) cudaEventDestroy(e1);

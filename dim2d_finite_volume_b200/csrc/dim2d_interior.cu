@@ -36,7 +36,8 @@ constexpr int SM_FX = 4 * TY * (TX + 1);
 constexpr int SM_FY = 4 * (TY + 1) * TX;
 constexpr int SM_DOUBLES = SM_RAW + SM_PRIM + SM_FX + SM_FY;
 
-// mode: 0 = write L(u) (time derivative), 1 = RK stage update,
+// Caller-provided layouts that the strip kernels cannot read (odd nx or
+// misaligned planes).  Mode 1 = RK stage update (periodic or open field),
 // 2 = L(u) of a buffer-layer grid: tiles over [box_x0, box_x1] x
 // [box_y0, box_y1], written where the grdpts_id map is interior_pt.  A face
 // whose stencil reaches a no_pt node (whatever it holds) feeds only points
@@ -44,7 +45,7 @@ constexpr int SM_DOUBLES = SM_RAW + SM_PRIM + SM_FX + SM_FY;
 // a boundary point of the layer.
 // Four 256-thread CTAs per SM (64 registers, no spills; 4 x 47.8 KB of shared
 // memory): with three, the face pass left the FP64 pipe waiting on latency.
-template <int MODE, bool WALL>
+template <int MODE>
 __global__ void __launch_bounds__(NT, 4) k_interior(StageArgs a) {
   extern __shared__ __align__(16) double sm[];
   double* sR = sm;
@@ -134,19 +135,7 @@ __global__ void __launch_bounds__(NT, 4) k_interior(StageArgs a) {
       fi.lap = d2n + d2t;
       fi.dtn = rdx * (fi.tb - fi.ta);
       fi.dkn = rdx * (fi.kb - fi.ka);
-      const int gxf = x0 + fx;  // face between columns gxf-1 and gxf
-      const bool w_face = WALL && a.wall_w && gxf == BC;
-      const bool e_face = WALL && a.wall_e && gxf == f.nx - BC;
-      if (w_face || e_face) {
-        // bc_operators_wall_xy_class.f:751-771: wall x-face; the low
-        // temperature is taken on the interior side (:473-490)
-        const int p = w_face ? pR : pL;
-        const double tl = k.c38cv * (sT[p] - k.iwe * sK[p]);
-        const double q = wall_heat_flux(a.wall, a.xmap0 + gxf * a.dx);
-        wall_face_flux(fi, tl, a.dx, q, w_face ? q : -q, k, F);
-      } else {
-        face_flux(fi, k, F);
-      }
+      face_flux(fi, k, F);
       const int o = fy * (TX + 1) + fx;
       sFx[o] = F[0];
       sFx[o + TY * (TX + 1)] = F[1];
@@ -180,18 +169,7 @@ __global__ void __launch_bounds__(NT, 4) k_interior(StageArgs a) {
       fi.lap = d2n + d2t;
       fi.dtn = rdy * (fi.tb - fi.ta);
       fi.dkn = rdy * (fi.kb - fi.ka);
-      const int gyf = y0 + gy;  // face between rows gyf-1 and gyf
-      const bool s_face = WALL && a.wall_s && gyf == BC;
-      const bool n_face = WALL && a.wall_n && gyf == f.ny - BC;
-      if (s_face || n_face) {
-        // bc_operators_wall_xy_class.f:729-749: wall y-face (:818-852)
-        const int p = s_face ? pT : pB;
-        const double tl = k.c38cv * (sT[p] - k.iwe * sK[p]);
-        const double q = wall_heat_flux(a.wall, a.xmap0 + (x0 + gx) * a.dx);
-        wall_face_flux(fi, tl, a.dy, q, s_face ? q : -q, k, F);
-      } else {
-        face_flux(fi, k, F);
-      }
+      face_flux(fi, k, F);
       const int o = gy * TX + gx;
       sFy[o] = F[0];
       sFy[o + (TY + 1) * TX] = F[2];      // momentum_x is tangential on a y-face
@@ -307,9 +285,7 @@ static cudaError_t set_smem_attr() {
   if (e != cudaSuccess) return e;
   if (dev >= 0 && dev < 64 && done[dev]) return cudaSuccess;
   const int bytes = (int)interior_smem_bytes();
-  const void* fns[5] = {(const void*)k_interior<0, false>, (const void*)k_interior<1, false>,
-                        (const void*)k_interior<0, true>, (const void*)k_interior<1, true>,
-                        (const void*)k_interior<2, false>};
+  const void* fns[2] = {(const void*)k_interior<1>, (const void*)k_interior<2>};
   for (const void* fn : fns) {
     e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     if (e != cudaSuccess) return e;
@@ -322,31 +298,27 @@ static cudaError_t set_smem_attr() {
   return cudaSuccess;
 }
 
-template <int MODE>
-static cudaError_t launch_mode(const StageArgs& a, cudaStream_t s) {
-  if (stage_uses_strip(a)) return launch_strip_stage(a, MODE, strip_shape_of(a), s);
+cudaError_t launch_interior_stage(const StageArgs& a, cudaStream_t s) {
+  if (strip_layout_ok(a)) return launch_strip_stage(a, 1, strip_shape_of(a), s);
+  if (a.mixed || a.wall_s) return cudaErrorInvalidValue;  // strips only
   cudaError_t e = set_smem_attr();
   if (e != cudaSuccess) return e;
   dim3 grid((a.f.nx - 2 * BC + TX - 1) / TX, (a.f.ny - 2 * BC + TY - 1) / TY);
-  if (a.wall_w || a.wall_e || a.wall_s || a.wall_n)
-    k_interior<MODE, true><<<grid, NT, interior_smem_bytes(), s>>>(a);
-  else
-    k_interior<MODE, false><<<grid, NT, interior_smem_bytes(), s>>>(a);
+  k_interior<1><<<grid, NT, interior_smem_bytes(), s>>>(a);
   return cudaGetLastError();
 }
 
-cudaError_t launch_interior_stage(const StageArgs& a, cudaStream_t s) {
-  return launch_mode<1>(a, s);
+// of a field that the library allocated: its layout suits the strips
+cudaError_t launch_time_dev(const StageArgs& a, cudaStream_t s) {
+  return launch_strip_stage(a, 0, strip_shape_of(a), s);
 }
-
-cudaError_t launch_time_dev(const StageArgs& a, cudaStream_t s) { return launch_mode<0>(a, s); }
 
 cudaError_t launch_time_dev_masked(const StageArgs& a, cudaStream_t s) {
   if (strip_layout_ok(a)) return launch_strip_masked(a, s);
   cudaError_t e = set_smem_attr();
   if (e != cudaSuccess) return e;
   dim3 grid((a.box_x1 - a.box_x0 + TX) / TX, (a.box_y1 - a.box_y0 + TY) / TY);
-  k_interior<2, false><<<grid, NT, interior_smem_bytes(), s>>>(a);
+  k_interior<2><<<grid, NT, interior_smem_bytes(), s>>>(a);
   return cudaGetLastError();
 }
 

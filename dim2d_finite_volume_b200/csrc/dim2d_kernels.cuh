@@ -115,8 +115,8 @@ struct StageArgs {
   double b;                        // stage weight: out = b*u0 + (1-b)*(uin + dt*L)
   int stage;                       // 1, 2, 3
   int periodic;                    // write periodic ghost images of edge cells
-  int wall_w, wall_e, wall_s, wall_n;  // wall flux override on that side
-  int variant;                         // 0 = 32x8 CTA tiles, 1..5 = warp strips (shape-1)
+  int wall_s;                      // the south side carries the wall's flux
+  int variant;                         // dim2d_set_variant
   int open;                            // OPEN_* mask of the time-integrated (Hedstrom)
                                        // ghost sections; strip launches integrate those
                                        // cells too (their first CTAs)
@@ -166,29 +166,37 @@ constexpr int TILE_Y = 8;
 size_t interior_smem_bytes();
 
 cudaError_t launch_interior_stage(const StageArgs& a, cudaStream_t s);
-// warp-streaming variant (dim2d_strip.cu); mode 0 = L(u), 1 = stage update;
-// shape 0..4 = strip height / warps per CTA (8,4) (16,4) (32,4) (16,8) (8,8)
+// strip kernel (dim2d_strip.cu); mode 0 = L(u), 1 = stage update; shape 0..4 =
+// strips of 8, 16, 32, 4, 2 rows, SHAPE_BY_SIZE = by the field's size
 cudaError_t launch_strip_stage(const StageArgs& a, int mode, int shape, cudaStream_t s);
-// The strip kernels read state rows as 16-byte pairs: they need an even
-// pitch and 16-byte aligned input planes (fields allocated by the library
-// always qualify; caller-provided layouts may not, and then use variant 0).
+// the ghost runs of open_runs_apart(a); launch_strip_stage follows on `s`
+cudaError_t launch_open_runs(const StageArgs& a, int mode, cudaStream_t s);
+// The strip kernels read state and u^n rows as 16-byte pairs: they need an
+// even pitch and 16-byte aligned planes.  Fields allocated by the library
+// always qualify; caller-provided layouts may not, and then run the tile
+// kernel (1024^2 periodic: 163 us per step there, 73 on strips).
 inline bool strip_layout_ok(const StageArgs& a) {
-  return a.f.pitch % 2 == 0 && reinterpret_cast<uintptr_t>(a.uin) % 16 == 0;
+  return a.f.pitch % 2 == 0 && reinterpret_cast<uintptr_t>(a.uin) % 16 == 0 &&
+         reinterpret_cast<uintptr_t>(a.u0) % 16 == 0;
 }
-// 1 if the stage launch of `a` runs a strip kernel (mixed precision always
-// does: the tile kernel has no FP32 face pass)
-inline bool stage_uses_strip(const StageArgs& a) {
-  return (a.variant > 0 || a.mixed) && strip_layout_ok(a);
-}
-// strip shape of a stage launch (variant 1..5; mixed fields on variant 0
-// use shape 1)
+// strip shape of a stage launch: variant 1..5, or by the field's size
+constexpr int SHAPE_BY_SIZE = -1;
 inline int strip_shape_of(const StageArgs& a) {
-  return a.variant >= 1 && a.variant <= 5 ? a.variant - 1 : (a.variant == 6 ? 3 : 1);
+  return a.variant >= 1 && a.variant <= 5 ? a.variant - 1 : SHAPE_BY_SIZE;
 }
-// 1 if the stage launch of `a` also covers the open-boundary ghost cells
-inline bool stage_fuses_open(const StageArgs& a) { return a.open && stage_uses_strip(a); }
-// variants 0..5 as above; 6 = the persistent kernel (a whole step per
-// launch, dim2d_persist.cu); its time derivative alone uses strip shape 3
+// 1 if the ghost cells of an open field take a launch of their own: tile
+// kernel, and variant 0 on hedstrom_xy, whose two kernels per stage callers
+// count (dim2d_launch_count); there the strips are a programmatic dependent
+// of the ghost launch and overlap it (launch_strip_stage)
+inline bool open_runs_apart(const StageArgs& a) {
+  return a.open == OPEN_ALL && a.variant == 0 && strip_layout_ok(a);
+}
+inline bool stage_fuses_open(const StageArgs& a) {
+  return a.open && strip_layout_ok(a) && !open_runs_apart(a);
+}
+// variants: 0 = strips of a height chosen by the field's size, 1..5 = strip
+// shapes 0..4, 6 = the persistent kernel (a whole step per launch,
+// dim2d_persist.cu; its time derivative alone runs as variant 0)
 constexpr int NUM_VARIANTS = 7;
 // L(a.uin) of the interior cells into a.uout (stage fields ignored)
 cudaError_t launch_time_dev(const StageArgs& a, cudaStream_t s);
@@ -264,7 +272,8 @@ struct BatchStageArgs {
 // ghost CTAs first; wall_S_reflection members have none)
 enum BatchKind : int { BK_PLAIN = 0, BK_WALL = 1, BK_OPEN = 2 };
 
-// one stage of every domain in P (shape as launch_strip_stage; mixed: the
+// one stage of every domain in P (shape as launch_strip_stage, by the size of
+// the whole launch; mixed: the
 // DIM2D_MIXED face pass for all of them); fills the CTA geometry fields of P.d
 cudaError_t launch_strip_batch(BatchStageArgs& P, int kind, int shape, bool mixed,
                                cudaStream_t s);

@@ -125,11 +125,18 @@ int check_status(dim2d_handle* h) {
 }
 
 cudaError_t launch_stage_work(dim2d_handle* h, const StageArgs& a, int mode) {
+  cudaError_t e = cudaSuccess;
+  const bool apart = open_runs_apart(a);
+  if (apart) {
+    e = launch_open_runs(a, mode, h->stream);
+    h->launches++;
+    if (e != cudaSuccess) return e;
+  }
   prof_begin(h);
-  cudaError_t e = mode == 0 ? launch_time_dev(a, h->stream) : launch_interior_stage(a, h->stream);
+  e = mode == 0 ? launch_time_dev(a, h->stream) : launch_interior_stage(a, h->stream);
   prof_end(h);
   h->launches++;
-  if (e == cudaSuccess && a.open && !stage_fuses_open(a)) {
+  if (e == cudaSuccess && a.open && !apart && !stage_fuses_open(a)) {
     e = launch_open_ghosts(a, mode, h->stream);
     h->launches++;
   }

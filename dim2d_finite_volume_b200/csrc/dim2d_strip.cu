@@ -786,9 +786,11 @@ __device__ __forceinline__ void strip_cta(const StageArgs& a, int b, int sx, int
 }
 
 // grid: [ghost CTAs (OPEN only)] + strip CTAs, one warp each
+// With `join`, a dependent of the launch before it that may start while that
+// runs and must not end before it: the first CTA sees to that.
 template <int MODE, int UN, bool OPEN, bool MIX>
 __global__ void __launch_bounds__(32, WARPS) k_strip(const __grid_constant__ StageArgs a,
-                                                    int ghost_ctas, int sx, int h) {
+                                                    int ghost_ctas, int sx, int h, int join) {
   int b = blockIdx.x;
   if (OPEN) {
     if (b < ghost_ctas) {
@@ -799,6 +801,14 @@ __global__ void __launch_bounds__(32, WARPS) k_strip(const __grid_constant__ Sta
     b -= ghost_ctas;
   }
   strip_cta<MODE, UN, MIX>(a, b, sx, h);
+  if (!OPEN && join && blockIdx.x == 0) wait_for_node_pass();
+}
+
+// the ghost runs alone (open_runs_apart)
+template <int MODE>
+__global__ void __launch_bounds__(32) k_open_runs(const __grid_constant__ StageArgs a) {
+  asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+  open_run<MODE>(a, blockIdx.x);
 }
 
 // stage arguments of domain i of a batched launch
@@ -818,7 +828,6 @@ __device__ __forceinline__ StageArgs batch_stage_args(const BatchStageArgs& P, i
   a.b = P.b;
   a.stage = P.stage;
   a.periodic = d.periodic;
-  a.wall_w = a.wall_e = a.wall_n = 0;
   a.wall_s = d.wall_s;
   a.variant = 0;
   a.open = d.open;
@@ -936,7 +945,6 @@ __device__ __forceinline__ StageArgs persist_stage_args(const PersistArgs& P, co
   a.b = st == 2 ? 0.75 : (st == 3 ? 1.0 / 3.0 : 0.0);  // rk3tvd_steps_module.f:225,444
   a.stage = st;
   a.periodic = d.periodic;
-  a.wall_w = a.wall_e = a.wall_n = 0;
   a.wall_s = d.wall_s;
   a.variant = 0;
   a.open = d.open;
@@ -1095,6 +1103,25 @@ inline cudaError_t launch_after_node_pass(const void* fn, unsigned blocks, cudaS
 
 // rows per strip of shape 0..4
 constexpr int SHAPE_ROWS[5] = {8, 16, 32, 4, 2};
+// Rows per strip by size: as few as still let every strip of the launch be
+// resident at once (148 SMs x 16 warps), since a stage then lasts as long as
+// one strip; 16 where even those do not fit (more rows leave the last wave
+// emptier, fewer repeat the two rows below a strip more often).  us per step:
+//   rows                       by size    2      4      8      16
+//   64^2 open                  10.3 (1)   12.3   14.3   18.4   28.7
+//   128^2 periodic             12.2 (1)   12.3   16.4   23.6   36.9
+//   301x187 half_wall_S_open   28.7 (2)   28.7   29.7   34.8   44.1
+//   512^2 wall_S_reflection    37.2 (4)   39.1   37.4   37.9   48.2
+//   1024^2 open                67.9 (16)  90.3   76.0   69.8   69.3
+//   1531x1117 periodic         115 (16)   148    122    114    115
+//   2048^2 open                228 (16)   325    261    239    230
+template <typename Strips>
+int rows_of(int shape, Strips strips) {
+  if (shape != SHAPE_BY_SIZE) return SHAPE_ROWS[shape];
+  int h = 1;
+  while (h < 16 && strips(h) > 148LL * WARPS) h *= 2;
+  return h;
+}
 template <int MODE, int UN, bool MIX>
 const void* strip_fn(bool open) {
   return open ? (const void*)k_strip<MODE, UN, true, MIX>
@@ -1138,8 +1165,13 @@ cudaError_t launch_batch_persistent(const PersistArgs& P, bool mixed, cudaStream
 cudaError_t launch_strip_batch(BatchStageArgs& P, int kind, int shape, bool mixed,
                                cudaStream_t s) {
   if (P.ndom <= 0) return cudaSuccess;
-  if (P.ndom > BATCH_MAX || shape < 0 || shape > 4) return cudaErrorInvalidValue;
-  int h = SHAPE_ROWS[shape];
+  if (P.ndom > BATCH_MAX || shape < SHAPE_BY_SIZE || shape > 4) return cudaErrorInvalidValue;
+  int h = rows_of(shape, [&](int rows) {
+    long long n = 0;
+    for (int i = 0; i < P.ndom; i++)
+      n += (long long)strips_across(P.d[i].f) * strips_up(P.d[i].f, rows);
+    return n;
+  });
   const bool open = kind == BK_OPEN || kind == BK_WALL;
   long long ghost = 0, strips = 0;
   bool pdl = false;
@@ -1162,30 +1194,37 @@ cudaError_t launch_strip_batch(BatchStageArgs& P, int kind, int shape, bool mixe
 
 // L(u) of a buffer-layer grid at its interior_pt points (MODE 2) over the
 // border box [box_x0, box_x1] x [box_y0, box_y1] (box_x0, box_y0 >= BC, so
-// every row and column read lies inside the grid).  Strips of 16 rows where
-// they fill the GPU's 148 x 16 warp slots, else of 8 rows for twice the
-// warps: layers are often thin bands.
+// every row and column read lies inside the grid).
 cudaError_t launch_strip_masked(const StageArgs& a, cudaStream_t s) {
   int sx = (a.box_x1 - (a.box_x0 & ~1) + SW) / SW;
   const int rows = a.box_y1 - a.box_y0 + 1;
-  int h = (long long)sx * ((rows + 15) / 16) >= 148LL * WARPS ? 16 : 8;
-  int ghost_ctas = 0;
+  int h = rows_of(SHAPE_BY_SIZE, [&](int r) { return (long long)sx * ((rows + r - 1) / r); });
+  int ghost_ctas = 0, join = 0;
   StageArgs aa = a;
-  void* args[] = {&aa, &ghost_ctas, &sx, &h};
+  void* args[] = {&aa, &ghost_ctas, &sx, &h, &join};
   return launch_after_node_pass(strip_fn<2, 0, false>(false), (unsigned)sx * (unsigned)((rows + h - 1) / h), s,
                                 false, args);
 }
 
 cudaError_t launch_strip_stage(const StageArgs& a, int mode, int shape, cudaStream_t s) {
-  if (shape < 0 || shape > 4) return cudaErrorInvalidValue;
-  int h = SHAPE_ROWS[shape], sx = strips_across(a.f);
-  int ghost_ctas = open_run_count(a.f, a.open);
-  const bool open = a.open != 0;
+  if (shape < SHAPE_BY_SIZE || shape > 4) return cudaErrorInvalidValue;
+  int sx = strips_across(a.f);
+  int h = rows_of(shape, [&](int rows) { return (long long)sx * strips_up(a.f, rows); });
+  int join = open_runs_apart(a);
+  int ghost_ctas = join ? 0 : open_run_count(a.f, a.open);
+  const bool open = ghost_ctas > 0;
   const void* fn = strip_fn(mode, a.stage != 1, open, a.mixed);
   StageArgs aa = a;
-  void* args[] = {&aa, &ghost_ctas, &sx, &h};
+  void* args[] = {&aa, &ghost_ctas, &sx, &h, &join};
   return launch_after_node_pass(fn, (unsigned)ghost_ctas + (unsigned)sx * (unsigned)strips_up(a.f, h),
-                                s, a.node_sides != 0, args);
+                                s, a.node_sides != 0 || join, args);
+}
+
+cudaError_t launch_open_runs(const StageArgs& a, int mode, cudaStream_t s) {
+  const unsigned n = (unsigned)open_run_count(a.f, a.open);
+  if (mode == 0) k_open_runs<0><<<n, 32, 0, s>>>(a);
+  else k_open_runs<1><<<n, 32, 0, s>>>(a);
+  return cudaGetLastError();
 }
 
 }  // namespace dim2d

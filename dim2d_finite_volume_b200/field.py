@@ -351,7 +351,8 @@ class Field:
 
     @property
     def variant(self):
-        """Stage-kernel variant in use (0 = CTA tiles, 1..5 = warp strips)."""
+        """Stage-kernel variant in use (0 = strips by the field's size,
+        1..5 = strips of 8, 16, 32, 4, 2 rows, 6 = persistent kernel)."""
         return library().dim2d_get_variant(self._h)
 
     @variant.setter

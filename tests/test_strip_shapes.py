@@ -65,3 +65,39 @@ def test_tiling_edges(oracle, F, preset, n, ny):
             if ref is not None:
                 a, b = got[v][rows], ref[v][rows]
                 assert np.abs(a - b).max() <= 1e-12 * np.abs(b).max(), (variant, v)
+
+
+@pytest.mark.parametrize("preset", ["periodic_xy", "hedstrom_xy"])
+@pytest.mark.parametrize("n,offset", [(60, 0), (60, 1), (61, 0)])
+def test_caller_layouts(F, preset, n, offset):
+    """dim2d_step_noalloc on the caller's array: even rows on a 16-byte boundary
+    (strips), the same off it, and odd rows (tiles) give the field's own
+    result (bar 1e-12, as in the no-allocation tests)."""
+    import ctypes
+
+    import torch
+    d = workloads.domain(n, 44, T0=0.95, bubbles=[(0.0, 0.0, 0.2)], mach=0.05, bc=preset, li=0.2)
+    with F.Field(d["nx"], d["ny"], bc=preset) as fld:
+        fld.ini(d["nodes"], d["x_map"], d["y_map"])
+        fld.integrate(d["dt"], 3)
+        ref = fld.download()
+    L = F.library()
+    L.dim2d_step_noalloc.argtypes = [ctypes.POINTER(F.Params), ctypes.c_int, ctypes.c_int,
+                                     ctypes.POINTER(ctypes.c_int), ctypes.POINTER(ctypes.c_int),
+                                     ctypes.POINTER(ctypes.c_int), ctypes.c_void_p, F._dp, F._dp,
+                                     ctypes.c_double, ctypes.c_int, ctypes.c_void_p]
+    arr = ctypes.c_int * 8
+    size = d["nodes"].size
+    buf = torch.zeros(size + 2, dtype=torch.float64, device="cuda")
+    dev = buf[offset:offset + size]
+    dev.copy_(torch.from_numpy(d["nodes"].reshape(-1)))
+    ch, ty, od = F._preset(preset)
+    rc = L.dim2d_step_noalloc(ctypes.byref(F.default_params()), d["nx"], d["ny"], arr(*ch),
+                              arr(*ty), arr(*od), ctypes.c_void_p(dev.data_ptr()),
+                              F._ptr(d["x_map"]), F._ptr(d["y_map"]), d["dt"], 3,
+                              ctypes.c_void_p(torch.cuda.current_stream().cuda_stream))
+    assert rc == 0
+    torch.cuda.synchronize()
+    got = dev.cpu().numpy().reshape(d["nodes"].shape)
+    for v in range(4):
+        assert np.abs(got[v] - ref[v]).max() <= 1e-12 * np.abs(ref[v]).max(), v
