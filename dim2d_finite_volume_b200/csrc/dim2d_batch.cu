@@ -6,14 +6,13 @@
 // borrows their device buffers.  Members are grouped by boundary kind:
 //   G_PERIODIC  periodic_xy            strip kernel writes the ghost images
 //   G_OPEN      hedstrom_xy            ghost cells fused into the launch
-//   G_WALL      wall_S_reflection,     strip kernel + node boundary pass; the
-//               wall_S_open,           open sections' ghost cells fused into
-//               half_wall_S_open       the launch
-//   G_MIRROR    reflection_xy          strip kernel + node boundary pass
+//   G_WALL      wall_S_reflection,     wall columns, mirror images and open
+//               wall_S_open,           sections by the launch
+//               half_wall_S_open
+//   G_MIRROR    reflection_xy          strip kernel writes the ghost images
 // and by precision (groups 4..7: the same kinds, DIM2D_MIXED fields).
-// One RK stage of a group is one batched launch over all its domains (plus
-// one batched node pass), so a step is at most 8 x 3 x 2 launches however
-// many domains there are.  The groups are independent: a captured step
+// One RK stage of a group is one batched launch over all its domains, so a
+// step is at most 8 x 3 launches however many domains there are.  The groups are independent: a captured step
 // graph holds one chain per group as parallel branches, so the kinds
 // overlap on the device.  Two graphs are kept, one per buffer parity
 // (which of A/B holds u^n), and rebuilt when members, dt or shapes change.
@@ -43,7 +42,6 @@ int kind_of(int g) {
   g %= NKINDS;
   return g == G_OPEN ? BK_OPEN : (g == G_WALL ? BK_WALL : BK_PLAIN);
 }
-bool has_node_pass(int g) { return g % NKINDS == G_WALL || g % NKINDS == G_MIRROR; }
 bool is_mixed(int g) { return g >= NKINDS; }
 }  // namespace
 
@@ -84,13 +82,12 @@ void drop_batch_graphs(dim2d_batch* b) {
   b->parity = 0;
 }
 
-// Stage `st` of the members of group g (indices idx): batched stage launch,
-// then the batched node pass.  in/out per stage: 1: A->B, 2: B->C, 3: C->B,
+// Stage `st` of the members of group g (indices idx), one batched launch per
+// BATCH_MAX of them.  in/out per stage: 1: A->B, 2: B->C, 3: C->B,
 // u^n = A.  dt_scale 0 gives the dry step of the autotuner.
 cudaError_t group_stage(dim2d_batch* b, int g, const std::vector<int>& idx, int st, int shape,
                         double dt_scale, cudaStream_t s) {
   static thread_local BatchStageArgs P;
-  static thread_local NodeBcBatchArgs Q;
   for (size_t c0 = 0; c0 < idx.size(); c0 += BATCH_MAX) {
     const int n = (int)std::min<size_t>(BATCH_MAX, idx.size() - c0);
     const dim2d_handle* h0 = b->m[idx[c0]];
@@ -99,9 +96,6 @@ cudaError_t group_stage(dim2d_batch* b, int g, const std::vector<int>& idx, int 
     P.stage = st;
     P.b = st == 2 ? 0.75 : (st == 3 ? 1.0 / 3.0 : 0.0);  // rk3tvd_steps_module.f:225,444
     P.ndom = n;
-    Q.k = h0->k;
-    Q.wall = h0->wall;
-    Q.ndom = n;
     for (int j = 0; j < n; j++) {
       const int i = idx[c0 + j];
       dim2d_handle* h = b->m[i];
@@ -122,32 +116,13 @@ cudaError_t group_stage(dim2d_batch* b, int g, const std::vector<int>& idx, int 
       d.wall_s = h->south_wall;
       d.open = h->open_mask;
       d.c = strip_coef_of(h->k, h->rdx, h->rdy);
-      d.node_sides = st >= 2 && has_node_pass(g) ? h->node_sides : 0;
-      NodeBcDomain& q = Q.d[j];
-      q.utmp = h->A;
-      q.u = out;
-      q.f = h->f;
-      q.dx = h->dx;
-      q.dy = h->dy;
-      q.rdx = h->rdx;
-      q.rdy = h->rdy;
-      q.xmap0 = h->xmap0;
-      q.ymap0 = h->ymap0;
-      q.south_wall = h->south_wall;
-      q.corners_y = h->corners_y;
-      q.open_w = h->open_w;
-      q.open_e = h->open_e;
-      q.open_n = h->open_n;
-      q.status = h->status;
+      d.mirror = h->mirror_sides;
+      d.wall_runs = h->south_wall ? wall_run_count(h->f, h->open_mask) : 0;
+      d.status = h->status;
     }
     cudaError_t e = launch_strip_batch(P, kind_of(g), shape, is_mixed(g), s);
     b->launches++;
     if (e != cudaSuccess) return e;
-    if (has_node_pass(g)) {
-      e = launch_node_bc_batch(Q, s);
-      b->launches++;
-      if (e != cudaSuccess) return e;
-    }
   }
   return cudaSuccess;
 }

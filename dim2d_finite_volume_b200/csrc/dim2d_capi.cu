@@ -253,12 +253,16 @@ int dim2d::create_field(const dim2d_params* p, int nx, int ny, const int bc_choi
   h->south_wall = south_wall;
   h->corners_y = corners_y;
   if (open) h->open_mask = OPEN_ALL;
-  if (mirrors) h->node_sides = NODE_W | NODE_E | NODE_S | NODE_N;
+  if (mirrors) {
+    h->node_sides = NODE_W | NODE_E | NODE_S | NODE_N;
+    h->mirror_sides = NODE_W | NODE_E | NODE_N | (south_wall ? 0 : NODE_S);
+  }
   if (open_wall) {
     h->open_n = h->open_e = 1;
     h->open_w = open_w;
     h->open_mask = OPEN_N | OPEN_E | OPEN_NE | (open_w ? OPEN_W | OPEN_NW : 0);
     h->node_sides = NODE_S | (open_w ? 0 : NODE_W);
+    h->mirror_sides = open_w ? 0 : NODE_W;
   }
   h->wall = make_wall(*p);
   std::memcpy(h->bc_choice, bc_choice, sizeof h->bc_choice);
@@ -537,8 +541,6 @@ int dim2d_autotune(dim2d_handle* h, int* chosen, double* times_ms) {
         const StageArgs a = make_stage_args(h, in[st - 1], out[st - 1], 0.0, st);
         cudaError_t r = launch_stage_work(h, a, 1);
         if (r != cudaSuccess) return r;
-        if (!h->periodic && !h->open_all && apply_bc_on_nodes(h, h->A, out[st - 1]))
-          return cudaErrorLaunchFailure;
       }
       return cudaSuccess;
     };

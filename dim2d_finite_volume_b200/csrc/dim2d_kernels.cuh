@@ -123,10 +123,12 @@ struct StageArgs {
   int mixed;                           // DIM2D_MIXED: FP32 face pass (strip kernels)
   double t;                            // field time (constant over the stages)
   double xmap0, ymap0;                 // x_map(1), y_map(1): x_map(i) = xmap0 + (i-1) dx
-  int node_sides;                      // NODE_* sides whose ghost cells the node pass just
-                                       // before this launch writes; non-zero: the launch is
-                                       // a programmatic dependent of that pass and the
-                                       // warps that read those ghosts wait for it
+  int mirror;                          // NODE_* mirror sides: the strips write their ghost
+                                       // images, as on a periodic field
+  int wall_runs;                       // south wall: runs of wall columns whose ghost cells
+                                       // the launch solves (wall_run_count)
+  unsigned int* status;                // wall root status word
+  int apart;                           // its ghost cells take the launch before (open_runs_apart)
   const int* __restrict__ mask;        // time derivative of a buffer-layer grid: its
                                        // grdpts_id map, written only where it is
                                        // interior_pt (1) inside [box_x0, box_x1] x
@@ -138,8 +140,40 @@ struct StageArgs {
   StripCoef<float> cf;                 // ... and their FP32 face pass (mixed)
 };
 
-// sides of StageArgs::node_sides
+// griddepcontrol: see dim2d_strip.cu
+#ifdef __CUDACC__
+__device__ __forceinline__ void let_dependents_start() {
+  asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+}
+__device__ __forceinline__ void wait_for_launch_before() {
+  asm volatile("griddepcontrol.wait;\n" ::: "memory");
+}
+// launch as a programmatic dependent of the launch before it on `s`
+inline cudaError_t launch_dependent(const void* fn, unsigned blocks, unsigned threads, size_t smem,
+                                    cudaStream_t s, void** args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(blocks);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelExC(&cfg, fn, args);
+}
+#endif
+
+// sides of a field: StageArgs::mirror, and what a node pass writes
 enum NodeSide : int { NODE_W = 1, NODE_E = 2, NODE_S = 4, NODE_N = 8 };
+// wall columns of the stage launch, by runs: one for the columns at each open
+// side, then the first of up to 29 interior columns, the others of 28
+// (dim2d_strip.cu)
+inline int wall_run_count(const Field& f, int open) {
+  return (open & OPEN_W ? 1 : 0) + (open & OPEN_E ? 1 : 0) +
+         (f.nx - 2 * BC - 1 + OPEN_RUN - 1) / OPEN_RUN;
+}
 
 // Node boundary pass of a field whose sides are mirrors (reflection_x/_y),
 // open (nothing to do) or, on the south side, the wall operator.
@@ -252,8 +286,9 @@ struct BatchDomain {
   double dx, dy, rdx, rdy, dt, xmap0;
   int periodic, wall_s;
   int open;                // OPEN_* mask of the time-integrated ghost sections
-  int node_sides;          // as StageArgs::node_sides
-  int ghost0, strip0, sx;  // first ghost CTA, first strip CTA, strips per row
+  int mirror, wall_runs;   // as StageArgs
+  unsigned int* status;
+  int edge0, strip0, sx;   // first edge CTA, first strip CTA, strips per row
   StripCoef<double> c;
 };
 
@@ -263,7 +298,7 @@ struct BatchStageArgs {
   int stage;
   double b;
   int ndom;
-  int ghost_ctas;  // total ghost CTAs (open and wall kinds), placed before all strips
+  int edge_ctas;   // edge runs of all domains, placed before all strips
   BatchDomain d[BATCH_MAX];
 };
 
@@ -277,27 +312,6 @@ enum BatchKind : int { BK_PLAIN = 0, BK_WALL = 1, BK_OPEN = 2 };
 // DIM2D_MIXED face pass for all of them); fills the CTA geometry fields of P.d
 cudaError_t launch_strip_batch(BatchStageArgs& P, int kind, int shape, bool mixed,
                                cudaStream_t s);
-
-struct NodeBcDomain {
-  const double* utmp;
-  double* u;
-  Field f;
-  double dx, dy, rdx, rdy, xmap0, ymap0;
-  int south_wall, corners_y;
-  int open_w, open_e, open_n;
-  unsigned int* status;
-  int cta0;
-};
-
-struct NodeBcBatchArgs {
-  DimConst k;
-  WallConst wall;
-  int ndom;
-  NodeBcDomain d[BATCH_MAX];
-};
-
-// node boundary pass of every domain in P; fills P.d[].cta0
-cudaError_t launch_node_bc_batch(NodeBcBatchArgs& P, cudaStream_t s);
 
 // ---- persistent batched kernel (dim2d_strip.cu): one launch advances
 // every domain of a batch (any mix of boundary kinds, one precision) by

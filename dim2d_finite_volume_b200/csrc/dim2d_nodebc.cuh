@@ -230,6 +230,54 @@ __host__ __device__ __forceinline__ double ld(const double* p, const Field& f, i
 
 }  // namespace
 
+// One wall column (compute_wall_S_ghost_cell, wall_xy_equilibrium_module.f:
+// 948-1040, with the temperature guess of bc_operators_wall_xy_class.f:
+// 898-930): what it reads and the ghost values it gives.
+struct WallIn {
+  double gr, gmx, gmy, gE;       // u^n at the first interior node (row 2)
+  double grw, gre, grs, grn;     // its density neighbours in u^n
+  double r1, mx1, my1, E1, r2;   // new state, rows 2 and (density) 3
+  double rw, re;                 // new density beside row 2
+};
+struct WallOut {
+  double r, r0, mx, my;  // ghost row 1: density, momenta; ghost row 0: density
+};
+// x = the column's coordinate; gt = WallGrad type of its tangential gradients
+__host__ __device__ __forceinline__ WallOut wall_column(const WallIn& in, int gt, double x,
+                                                        double dx, double dy,
+                                                        const WallConst& wall, const DimConst& k,
+                                                        unsigned int* status) {
+  // temperature guess, temperature_eff dim2d_prim_module.f:652-691
+  double gx;
+  if (gt == WG_L0) gx = 1.0 / dx * (-in.gr + in.gre);
+  else if (gt == WG_R0) gx = 1.0 / dx * (-in.grw + in.gr);
+  else gx = 0.5 / dx * (-in.grw + in.gre);
+  const double gy = 0.5 / dy * (-in.grs + in.grn);
+  const double vx = in.gmx / in.gr, vy = in.gmy / in.gr;
+  const double teff = 1.0 / in.gr * (in.gE - 0.5 * in.gr * (vx * vx + vy * vy) -
+                                     0.5 / k.we * (gx * gx + gy * gy) + 3.0 * (in.gr * in.gr));
+  const double Tg = 3.0 / (8.0 * k.cv_r) * teff;
+  WallRoot c;
+  c.md1 = in.r1;
+  c.md2 = in.r2;
+  c.my0 = in.rw;
+  c.my1 = in.re;
+  c.gt = gt;
+  c.vx = -in.my1 / in.r1;
+  c.vy = in.mx1 / in.r1;
+  c.Ed = in.E1;
+  c.dxn = dy;
+  c.dyt = dx;
+  c.q = wall_heat_flux(wall, x);
+  c.cosang = wall.cos_angle;
+  WallOut o;
+  o.r = wall_root(c, Tg, in.grs, k, status);
+  o.r0 = in.r2 + 3.0 * (-in.r1 + o.r);   // :1439-1465 (high-order extrapolation)
+  o.mx = -1.0 * in.mx1 / in.r1 * o.r;    // sign_trans
+  o.my = 1.0 * in.my1 / in.r1 * o.r;     // sign_normal
+  return o;
+}
+
 // Work items of the node pass, in order: W mirror cells, E mirror cells,
 // N mirror cells (each only where that side is a mirror), S cells (wall
 // columns or mirror cells), then the corner cells that have node work.
@@ -315,52 +363,32 @@ __host__ __device__ inline void node_bc_cell(const NodeBcArgs& a, int m) {
     // tangential gradients (gradient_x_x_oneside_L0/R0 and GT_L0/GT_R0,
     // bc_operators_wall_xy_class.f:340-360)
     const int gt = x == 0 ? WG_L0 : (x == nx - 1 ? WG_R0 : WG_CENTRED);
-    // temperature guess from u^n at the first interior node
-    // (bc_operators_wall_xy_class.f:898-930, temperature_eff
-    // dim2d_prim_module.f:652-691)
-    double Tg;
-    {
-      const double r = ld(a.utmp, f, 0, x, 2);
-      const double mx = ld(a.utmp, f, 1, x, 2), my = ld(a.utmp, f, 2, x, 2);
-      const double E = ld(a.utmp, f, 3, x, 2);
-      double gx;
-      if (gt == WG_L0) gx = 1.0 / a.dx * (-ld(a.utmp, f, 0, x, 2) + ld(a.utmp, f, 0, x + 1, 2));
-      else if (gt == WG_R0) gx = 1.0 / a.dx * (-ld(a.utmp, f, 0, x - 1, 2) + ld(a.utmp, f, 0, x, 2));
-      else gx = 0.5 / a.dx * (-ld(a.utmp, f, 0, x - 1, 2) + ld(a.utmp, f, 0, x + 1, 2));
-      const double gy = 0.5 / a.dy * (-ld(a.utmp, f, 0, x, 1) + ld(a.utmp, f, 0, x, 3));
-      const double vx = mx / r, vy = my / r;
-      const double teff = 1.0 / r * (E - 0.5 * r * (vx * vx + vy * vy) -
-                                     0.5 / k.we * (gx * gx + gy * gy) + 3.0 * (r * r));
-      Tg = 3.0 / (8.0 * k.cv_r) * teff;
-    }
-    const double md_guess = ld(a.utmp, f, 0, x, 1);
-    // compute_wall_S_ghost_cell, wall_xy_equilibrium_module.f:948-1040
-    const double r1 = ld(u, f, 0, x, 2), r2 = ld(u, f, 0, x, 3);
-    const double mx1 = ld(u, f, 1, x, 2), my1 = ld(u, f, 2, x, 2);
-    WallRoot c;
-    c.md1 = r1;
-    c.md2 = r2;
-    // md_y: neighbours of the first interior node.  A mirror W/E ghost is
-    // read at its source (the mirror side comes before S in the presets'
-    // order and is written by this same launch); an open side's ghost
-    // column holds the stage output.  The one-sided types read one side.
-    c.my0 = c.my1 = 0.0;
+    WallIn in{};
+    in.gr = ld(a.utmp, f, 0, x, 2);
+    in.gmx = ld(a.utmp, f, 1, x, 2);
+    in.gmy = ld(a.utmp, f, 2, x, 2);
+    in.gE = ld(a.utmp, f, 3, x, 2);
+    if (gt != WG_L0) in.grw = ld(a.utmp, f, 0, x - 1, 2);
+    if (gt != WG_R0) in.gre = ld(a.utmp, f, 0, x + 1, 2);
+    in.grs = ld(a.utmp, f, 0, x, 1);
+    in.grn = ld(a.utmp, f, 0, x, 3);
+    in.r1 = ld(u, f, 0, x, 2);
+    in.r2 = ld(u, f, 0, x, 3);
+    in.mx1 = ld(u, f, 1, x, 2);
+    in.my1 = ld(u, f, 2, x, 2);
+    in.E1 = ld(u, f, 3, x, 2);
+    // neighbours of the first interior node.  A mirror W/E ghost is read at
+    // its source (the mirror side comes before S in the presets' order and is
+    // written by this same launch); an open side's ghost column holds the
+    // stage output.  The one-sided types read one side.
     if (gt != WG_L0)
-      c.my0 = x - 1 < BC && !a.open_w ? ld(u, f, 0, mirror_lo_hi(x - 1, nx), 2)
+      in.rw = x - 1 < BC && !a.open_w ? ld(u, f, 0, mirror_lo_hi(x - 1, nx), 2)
                                       : ld(u, f, 0, x - 1, 2);
     if (gt != WG_R0)
-      c.my1 = x + 1 >= nx - BC && !a.open_e ? ld(u, f, 0, mirror_lo_hi(x + 1, nx), 2)
+      in.re = x + 1 >= nx - BC && !a.open_e ? ld(u, f, 0, mirror_lo_hi(x + 1, nx), 2)
                                             : ld(u, f, 0, x + 1, 2);
-    c.gt = gt;
-    c.vx = -my1 / r1;
-    c.vy = mx1 / r1;
-    c.Ed = ld(u, f, 3, x, 2);
-    c.dxn = a.dy;
-    c.dyt = a.dx;
-    c.q = wall_heat_flux(a.wall, a.xmap0 + x * a.dx);
-    c.cosang = a.wall.cos_angle;
     unsigned int st = 0;
-    const double rg = wall_root(c, Tg, md_guess, k, &st);
+    const WallOut o = wall_column(in, gt, a.xmap0 + x * a.dx, a.dx, a.dy, a.wall, k, &st);
     if (st && a.status) {
 #ifdef __CUDA_ARCH__
       atomicOr(a.status, st);
@@ -368,9 +396,7 @@ __host__ __device__ inline void node_bc_cell(const NodeBcArgs& a, int m) {
       *a.status |= st;
 #endif
     }
-    const double rg2 = r2 + 3.0 * (-r1 + rg);      // :1439-1465 (high-order extrapolation)
-    const double mxg = -1.0 * mx1 / r1 * rg;        // sign_trans
-    const double myg = 1.0 * my1 / r1 * rg;         // sign_normal
+    const double rg = o.r, rg2 = o.r0, mxg = o.mx, myg = o.my;
     NBC_ST(&u[(size_t)1 * f.pitch + x], rg);
     NBC_ST(&u[(size_t)0 * f.pitch + x], rg2);
     NBC_ST(&u[f.plane + (size_t)1 * f.pitch + x], mxg);

@@ -5,9 +5,7 @@
 // C = 3/4 A + 1/4 (B + dt L(B)); stage 3 writes B = 1/3 A + 2/3 (C + dt L(C));
 // then A and B swap.  u^n stays intact in A until the last boundary pass,
 // which the wall operator reads as nodes_tmp (bc_operators_wall_xy_class.f).
-// Each stage is followed by the node boundary pass; for periodic fields the
-// stage kernel writes the ghost images itself, for open fields a second
-// kernel integrates the ghost cells.
+// A stage launch sets the ghost cells of its output itself (stage()).
 #include <utility>
 
 #include "dim2d_internal.h"
@@ -36,9 +34,10 @@ StageArgs make_stage_args(const dim2d_handle* h, const double* uin, double* uout
   a.t = h->t;
   a.xmap0 = h->xmap0;
   a.ymap0 = h->ymap0;
-  // stages 2 and 3 follow the node pass of the stage before (stage()): they
-  // may start while it runs, only the warps that read its ghosts wait
-  a.node_sides = st >= 2 ? h->node_sides : 0;
+  a.mirror = h->mirror_sides;
+  a.wall_runs = h->south_wall ? wall_run_count(h->f, h->open_mask) : 0;
+  a.status = h->status;
+  a.apart = open_runs_apart(a);
   a.wall = h->wall;
   a.k = h->k;
   a.c = strip_coef_of(h->k, h->rdx, h->rdy);
@@ -126,7 +125,7 @@ int check_status(dim2d_handle* h) {
 
 cudaError_t launch_stage_work(dim2d_handle* h, const StageArgs& a, int mode) {
   cudaError_t e = cudaSuccess;
-  const bool apart = open_runs_apart(a);
+  const bool apart = a.apart != 0;
   if (apart) {
     e = launch_open_runs(a, mode, h->stream);
     h->launches++;
@@ -144,14 +143,12 @@ cudaError_t launch_stage_work(dim2d_handle* h, const StageArgs& a, int mode) {
 }
 
 static int stage(dim2d_handle* h, int st, const double* uin, double* uout, double dt) {
-  // on open fields every ghost cell has a time derivative and is integrated
-  // like the interior (x/y_borders widened, field_abstract_class.f:244-270)
-  // and no node boundary pass follows; the mixed presets integrate their
-  // open sections and run the node pass for the others
+  // The stage launch leaves the ghost cells of its output set: periodic and
+  // mirror images by the strips, open sections integrated like the interior
+  // (x/y_borders widened, field_abstract_class.f:244-270), wall columns by
+  // their runs.
   cudaError_t e = launch_stage_work(h, make_stage_args(h, uin, uout, dt, st), 1);
-  if (e != cudaSuccess) return cuda_error(e, "rk3 stage");
-  if (h->periodic || h->open_all) return DIM2D_OK;  // periodic images: by the stage kernel
-  return apply_bc_on_nodes(h, h->A, uout);
+  return e == cudaSuccess ? DIM2D_OK : cuda_error(e, "rk3 stage");
 }
 
 int rk3_step(dim2d_handle* h, double dt) {

@@ -52,21 +52,14 @@ namespace {
 constexpr int SW = STRIP_COLS;  // cells per strip
 constexpr int WARPS = 16;       // resident warps per SM (one warp per CTA, <= 128 registers)
 
-// A stage launched as a programmatic dependent of the node pass before it
-// (StageArgs::node_sides != 0) starts while that pass runs: a warp whose
-// rows or columns reach a side the pass writes waits for the pass (and its
-// memory) before its first read; the other warps read only cells the
-// previous stage wrote, complete before the pass began.
-__device__ __forceinline__ void wait_for_node_pass() {
-  asm volatile("griddepcontrol.wait;\n" ::: "memory");
-}
-// 1 if the warp's reads -- columns c0-2 .. c0+31, rows y0-2 .. y1+1,
-// clamped to the field -- reach a ghost cell of the sides in `sides`
-__device__ __forceinline__ bool reads_node_ghosts(int sides, const Field& f, int c0, int y0,
-                                                  int y1) {
-  return ((sides & NODE_W) && c0 - 2 < BC) || ((sides & NODE_E) && c0 + 31 >= f.nx - BC) ||
-         ((sides & NODE_S) && y0 - 2 < BC) || ((sides & NODE_N) && y1 + 1 >= f.ny - BC);
-}
+// Every launch of a step is a programmatic dependent of the one before it on
+// its stream: it lets its own dependent start before it ends and waits for the
+// launch before it, complete and visible, before its first read
+// (griddepcontrol.wait), so that launch latency and block scheduling overlap
+// that launch's end.  Strips after their own ghost runs (StageArgs::apart)
+// start without waiting: the runs have themselves waited for the launch whose
+// output both read before they let the strips start, and write other cells;
+// the first CTA waits at its end, so that the strips' end implies the runs'.
 
 template <typename T>
 __device__ __forceinline__ T from_left(T v) {
@@ -101,6 +94,7 @@ __device__ __forceinline__ void cp_async_wait() {
 constexpr int RC = 34, NS = 5, NU = 3;
 constexpr int ST_ROW = 4 * RC, UN_ROW = ST_ROW;
 constexpr int WARP_DOUBLES = NS * ST_ROW + NU * UN_ROW;
+constexpr int KEEP_AT = ST_ROW;  // what a wall run keeps (strip_warp)
 extern __shared__ __align__(16) double g_ring[];
 
 // The lane's part in copying a row: 16-byte pairs of columns c0-2 .. c0+29
@@ -392,42 +386,40 @@ __device__ __forceinline__ double pressure(const NodeUV& n, double r, double mx,
   return fma(mul(k.c15cv * r, n.inv), w + w, m3r2);
 }
 
-// L(u) (MODE 0) or stage update (MODE 1) of one ghost cell at offset o
+// L(u) (MODE 0) or stage update (MODE 1) of a ghost cell: q its state, L its
+// time derivative (in place)
 template <int MODE>
-__device__ __forceinline__ void store_ghost(const StageArgs& a, size_t o, const double q[4],
-                                            double L[4], const double un[4]) {
+__device__ __forceinline__ void update_ghost(const StageArgs& a, const double q[4], double L[4],
+                                             const double un[4]) {
   if (a.k.gravity_ac) {  // openbc_operators_module.f:354-372
     L[2] = fma(-q[0], a.k.gravity, L[2]);
     L[3] = fma(-q[2], a.k.gravity, L[3]);
   }
+  if (MODE == 1) {
 #pragma unroll
-  for (int v = 0; v < 4; v++) {
-    double out = L[v];
-    if (MODE == 1) {
-      out = fma(a.dt, L[v], q[v]);
-      if (a.stage != 1) out = fma(a.b, un[v], (1.0 - a.b) * out);
+    for (int v = 0; v < 4; v++) {
+      L[v] = fma(a.dt, L[v], q[v]);
+      if (a.stage != 1) L[v] = fma(a.b, un[v], (1.0 - a.b) * L[v]);
     }
-    a.uout[o + v * a.f.plane] = out;
   }
 }
 
-// One ghost layer (0 inner, 1 outer) of `count` <= OPEN_RUN cells from position
-// `first` along edge `side` (0..3 = S, N, W, E).  Lane l holds position first-2+l; cells are
-// lanes 2 .. count+1, faces lanes 2 .. count+2.  Inner layer: the interior
-// operators across the edge; outer layer: the one-sided ones (the *_L0 / *_R0
-// sets, bc_operators_openbc_normal_class.f:563-713), whose second derivative
-// across the edge is the inner layer's.
+// The ghost cell at position s along edge `side` (0..3 = S, N, W, E) in the
+// inner or outer layer, from the lanes that hold the positions beside it (lane
+// l-1 and l+1): its offset, and L(u) or new state in out.  Inner layer: the
+// interior operators across the edge; outer layer: the one-sided ones (the
+// *_L0 / *_R0 sets, bc_operators_openbc_normal_class.f:563-713), whose second
+// derivative across the edge is the inner layer's.  All lanes take part.
 template <int MODE>
-__device__ __forceinline__ void open_edge_run(const StageArgs& a, int side, int layer, int first,
-                                              int count) {
-  const int lane = threadIdx.x & 31;
+__device__ __forceinline__ size_t open_edge_cell(const StageArgs& a, int side, int s, bool outer,
+                                                 double out[4]) {
   const Field& f = a.f;
   const DimConst& k = a.k;
   const bool ye = side >= 2, hi = side & 1;  // edge along y; N or E
   const size_t along = ye ? f.pitch : 1, across = ye ? 1 : f.pitch;
   const int na = ye ? f.ny : f.nx, nc = ye ? f.nx : f.ny;
   const int c0 = hi ? nc - 3 : 0;  // the three nodes across: c0, c0+1, c0+2
-  const size_t o0 = min(max(first - 2 + lane, 0), na - 1) * along + c0 * across;
+  const size_t o0 = min(max(s, 0), na - 1) * along + c0 * across;
   const size_t V = f.plane, vs = ye ? 2 * V : V, vc = ye ? V : 2 * V;
   double r[3], ms[3], mc[3], e[3], un[4];
 #pragma unroll
@@ -438,7 +430,6 @@ __device__ __forceinline__ void open_edge_run(const StageArgs& a, int side, int 
     mc[j] = __ldcg(p + vc);
     e[j] = __ldcg(p + 3 * V);
   }
-  const bool outer = layer == 1;
   const int jl = outer ? (hi ? 2 : 0) : 1;  // the layer's node
   const size_t o = o0 + jl * across;
 #pragma unroll
@@ -480,18 +471,12 @@ __device__ __forceinline__ void open_edge_run(const StageArgs& a, int side, int 
              twice(n[0].v, n[1].v, n[2].v), ca.th);
   double F[3], F3;
   face2(fs, ca, a.c.s, F, &F3);
-  if (ye && a.wall_s && first == BC) {
+  if (ye && a.wall_s && s == BC) {
     // the face under the first interior row carries the wall corner's flux
     // (bc_operators_wall_xy_class.f:702-854)
-    double W[3], W3;
-    wall_face2(fs, ca, q.th, a.dy, wall_heat_flux(a.wall, a.xmap0 + (c0 + jl) * a.dx), k, W, &W3);
-    if (lane == 2) {
-      F[0] = W[0];
-      F[1] = W[1];
-      F[2] = W[2];
-      F3 = W3;
-    }
+    wall_face2(fs, ca, q.th, a.dy, wall_heat_flux(a.wall, a.xmap0 + (c0 + jl) * a.dx), k, F, &F3);
   }
+  __syncwarp();
   double D[4];
 #pragma unroll
   for (int v = 0; v < 3; v++) D[v] = F[v] - from_right(F[v]);
@@ -501,12 +486,34 @@ __device__ __forceinline__ void open_edge_run(const StageArgs& a, int side, int 
                 rdc * side_diff(n[0].u, n[1].u, n[2].u),
                 rdc * side_diff(n[0].v, n[1].v, n[2].v), rdc * side_diff(p[0], p[1], p[2]), hi, k,
                 ch);
-  if (lane >= 2 && lane < 2 + count) {
-    const double h = 0.5 * rda;
-    const double qc[4] = {rl, ye ? mcl : msl, ye ? msl : mcl, el};
-    double L[4] = {fma(h, D[0], ch[0]), ye ? fma(h, D[2], ch[2]) : fma(h, D[1], ch[1]),
-                   ye ? fma(h, D[1], ch[1]) : fma(h, D[2], ch[2]), fma(h, D[3], ch[3])};
-    store_ghost<MODE>(a, o, qc, L, un);
+  const double h = 0.5 * rda;
+  const double qc[4] = {rl, ye ? mcl : msl, ye ? msl : mcl, el};
+  out[0] = fma(h, D[0], ch[0]);
+  out[1] = ye ? fma(h, D[2], ch[2]) : fma(h, D[1], ch[1]);
+  out[2] = ye ? fma(h, D[1], ch[1]) : fma(h, D[2], ch[2]);
+  out[3] = fma(h, D[3], ch[3]);
+  update_ghost<MODE>(a, qc, out, un);
+  return o;
+}
+
+// One ghost layer (0 inner, 1 outer) of `count` <= OPEN_RUN cells from position
+// `first` along edge `side`.  Lane l holds position first-2+l; cells are lanes
+// 2 .. count+1, faces lanes 2 .. count+2.
+template <int MODE>
+__device__ __forceinline__ void open_edge_run(const StageArgs& a, int side, int layer, int first,
+                                              int count) {
+  const int lane = threadIdx.x & 31, s = first - 2 + lane;
+  double q[4];
+  const size_t o = open_edge_cell<MODE>(a, side, s, layer == 1, q);
+  if (lane < 2 || lane >= 2 + count) return;
+  double* out = a.uout + o;
+#pragma unroll
+  for (int v = 0; v < 4; v++) out[v * a.f.plane] = q[v];
+  // half_wall_S_open's NW corner mirrors the open N ghost rows
+  if (MODE == 1 && side == 1 && s < 2 * BC && (a.mirror & NODE_W)) {
+    out += 2 * BC - 1 - 2 * s;
+#pragma unroll
+    for (int v = 0; v < 4; v++) out[v * a.f.plane] = v == 1 ? -q[v] : q[v];
   }
 }
 
@@ -549,13 +556,16 @@ __device__ __forceinline__ void open_corner_cells(const StageArgs& a, int mask) 
   L[1] = cx[2] + cy[1];
   L[2] = cx[1] + cy[2];
   L[3] = cx[3] + cy[3];
-  store_ghost<MODE>(a, o, q[0], L, un);
+  update_ghost<MODE>(a, q[0], L, un);
+#pragma unroll
+  for (int v = 0; v < 4; v++) a.uout[o + v * V] = L[v];
 }
 
 // ghost run number m of a launch: the runs of the open edges S, N, W, E, then
 // one for the corners
 template <int MODE>
 __device__ __forceinline__ void open_run(const StageArgs& a, int m) {
+  wait_for_launch_before();
   for (int side = 0; side < 4; side++) {
     if (!(a.open >> side & 1)) continue;
     const int cells = (side < 2 ? a.f.nx : a.f.ny) - 2 * BC;
@@ -572,9 +582,13 @@ __device__ __forceinline__ void open_run(const StageArgs& a, int m) {
 
 // The strip of one warp: columns c0 .. c0+29 (interior ones), rows y0 ..
 // y1-1.
-// UN: whether the stage reads u^n (stages 2 and 3), 2: by a.stage.
-template <int MODE, int UN, bool MIX>
-__device__ __forceinline__ void strip_warp(const StageArgs& a, int c0, int y0, int y1) {
+// UN: whether the stage reads u^n (stages 2 and 3), 2: by a.stage (persistent
+// kernel: no images of mirrors).  KEEP: the launch has wall runs; with `keep`
+// (two rows) nothing is stored, and the new state of row y0 and the new
+// density of row y0+1 stay in the lane's places of the ring (KEEP_AT).
+template <int MODE, int UN, bool MIX, bool KEEP = false>
+__device__ __forceinline__ void strip_warp(const StageArgs& a, int c0, int y0, int y1,
+                                           bool keep = false) {
   using T = typename FaceType<MIX>::type;
   const int lane = threadIdx.x & 31;
   const Field f = a.f;
@@ -582,7 +596,7 @@ __device__ __forceinline__ void strip_warp(const StageArgs& a, int c0, int y0, i
   const StripCoef<T>& c = coef_of(a, T(0));
   const bool need_un = MODE == 1 && (UN == 2 ? a.stage != 1 : UN == 1);
 
-  if (a.node_sides && reads_node_ghosts(a.node_sides, f, c0, y0, y1)) wait_for_node_pass();
+  if (UN != 2 && !a.apart) wait_for_launch_before();
 
   // the lane's column (columns past the field are not stored); its place in
   // a ring row
@@ -642,12 +656,16 @@ __device__ __forceinline__ void strip_warp(const StageArgs& a, int c0, int y0, i
 
   const bool active = lane >= 1 && lane <= SW && x <= f.nx - 1 - BC &&
                       (MODE != 2 || (x >= a.box_x0 && x <= a.box_x1));
+  // column of the cell's image in a ghost layer of a periodic or mirror side
+  const bool images = MODE == 1 && (a.periodic || (UN != 2 && a.mirror));
   int ix2 = -1;
-  if (MODE == 1 && a.periodic) {
-    const int px = f.nx - 2 * BC;
-    if (x < 2 * BC) ix2 = x + px;
-    else if (x >= f.nx - 2 * BC) ix2 = x - px;
+  if (images) {
+    if (x < 2 * BC && (a.periodic || (a.mirror & NODE_W)))
+      ix2 = a.periodic ? x + f.nx - 2 * BC : 2 * BC - 1 - x;
+    else if (x >= f.nx - 2 * BC && (a.periodic || (a.mirror & NODE_E)))
+      ix2 = a.periodic ? x - (f.nx - 2 * BC) : 2 * (f.nx - BC) - 1 - x;
   }
+  const bool column_images = images && __any_sync(0xffffffffu, ix2 >= 0);
   // stage update: out = b u^n + (1 - b) (u + dt L), L from doubled fluxes
   const double w = MODE == 1 ? (1.0 - a.b) * a.dt : 1.0;
   const double wx = 0.5 * a.rdx * w, wy = 0.5 * a.rdy * w;
@@ -702,6 +720,12 @@ __device__ __forceinline__ void strip_warp(const StageArgs& a, int c0, int y0, i
     const NodeQ<T> n1 =
         node<T>(uv, r1, mx1, my1, e1, r1 - s1[-1], s1[1] - r1, dn0, dn1, cd);
 
+    // the dependent launch may start (on its last row: its warps then find
+    // every SM about as empty as the others; let in at the start of this
+    // launch, they crowd the SMs that finish first: 1024^2 open 71.7 us per
+    // step, 67.7 so)
+    if (UN != 2 && y == y1 - 1) let_dependents_start();
+
     // y-face between rows y and y+1
     const T ul1 = from_left(n1.u), vl1 = from_left(n1.v);
     const T gxu1 = from_right(n1.u) - ul1, gxv1 = from_right(n1.v) - vl1;
@@ -723,22 +747,34 @@ __device__ __forceinline__ void strip_warp(const StageArgs& a, int c0, int y0, i
       q[2] = fma(-w, r0 * a.k.gravity, q[2]);
       q[3] = fma(-w, my0 * a.k.gravity, q[3]);
     }
+    if (KEEP && keep) {
+      // (slots 1 and 2, of rows y0-1 and y0, are free after the prologue)
+#pragma unroll
+      for (int v = 0; v < 4; v++) ring[KEEP_AT + (y - y0) * ST_ROW + v * 32 + lane] = q[v];
+    }
     // MODE 2 writes the interior_pt points of the layer map only
-    if (active && (MODE != 2 || __ldg(a.mask + (size_t)y * P + x) == 1)) {
+    else if (active && (MODE != 2 || __ldg(a.mask + (size_t)y * P + x) == 1)) {
 #pragma unroll
       for (int v = 0; v < 4; v++) out[v * V] = q[v];
-      if (MODE == 1 && a.periodic) {  // periodic_xy/bc_operators_class.f:156-199
+      // periodic_xy/bc_operators_class.f:156-199; mirrors change the sign of
+      // the normal momentum (bc_operators_reflection_{x,y}_class.f:178-296)
+      if (images && (column_images || y < 2 * BC || y >= f.ny - 2 * BC)) {
         int iy2 = -1;
-        const int py = f.ny - 2 * BC;
-        if (y < 2 * BC) iy2 = y + py;
-        else if (y >= f.ny - 2 * BC) iy2 = y - py;
+        if (y < 2 * BC && (a.periodic || (a.mirror & NODE_S)))
+          iy2 = a.periodic ? y + f.ny - 2 * BC : 2 * BC - 1 - y;
+        else if (y >= f.ny - 2 * BC && (a.periodic || (a.mirror & NODE_N)))
+          iy2 = a.periodic ? y - (f.ny - 2 * BC) : 2 * (f.ny - BC) - 1 - y;
+        if (ix2 >= 0 || iy2 >= 0) {
+          const double mx = a.periodic ? q[1] : -q[1], my = a.periodic ? q[2] : -q[2];
 #pragma unroll
-        for (int v = 0; v < 4; v++) {
-          double* dst = a.uout + v * V;
-          if (ix2 >= 0) dst[(size_t)y * P + ix2] = q[v];
-          if (iy2 >= 0) {
-            dst[(size_t)iy2 * P + x] = q[v];
-            if (ix2 >= 0) dst[(size_t)iy2 * P + ix2] = q[v];
+          for (int v = 0; v < 4; v++) {
+            double* dst = a.uout + v * V;
+            const double qx = v == 1 ? mx : q[v], qy = v == 2 ? my : q[v];
+            if (ix2 >= 0) dst[(size_t)y * P + ix2] = qx;
+            if (iy2 >= 0) {
+              dst[(size_t)iy2 * P + x] = qy;
+              if (ix2 >= 0) dst[(size_t)iy2 * P + ix2] = v == 1 ? mx : qy;
+            }
           }
         }
       }
@@ -773,41 +809,166 @@ __device__ __forceinline__ void strip_warp(const StageArgs& a, int c0, int y0, i
   __syncwarp();
 }
 
-// The strip of CTA number b of one field (one warp per CTA): sx strips per
-// band of h rows, x fastest.
-template <int MODE, int UN, bool MIX>
-__device__ __forceinline__ void strip_cta(const StageArgs& a, int b, int sx, int h) {
-  // MODE 2 (buffer-layer grid): strips over the border box, the first one
-  // starting at an even column so that the rows' 16-byte pairs stay aligned
-  const int c0 = (MODE == 2 ? (a.box_x0 & ~1) : BC) + (b % sx) * SW;
-  const int y0 = (MODE == 2 ? a.box_y0 : BC) + (b / sx) * h;
-  const int ylast = MODE == 2 ? a.box_y1 : a.f.ny - BC - 1;
-  strip_warp<MODE, UN, MIX>(a, c0, y0, min(y0 + h, ylast + 1));
+// Wall run m of a field with a south wall: the ghost cells of up to 29 wall
+// columns (the first of the interior runs) or 28, or of the wall corner at an
+// open side: its two ghost columns and the interior column beside them.  The
+// warp evaluates the new state of the two rows above the columns as the strips
+// do, without storing it (in an open side's ghost columns as the ghost runs
+// do), and solves each column's root from its lanes, so that no pass over the
+// stage's output has to follow it: before, a launch of its own stood between
+// two stages, some 5 us on small fields.  The runs take the first CTAs of the
+// grid; their dependent evaluations overlap the strips.
+// The rows are evaluated by the strips' own code (strip_warp with `keep`): a
+// copy of it for the runs cost the strips of the same kernel 10 % by its
+// register allocation (wall_S_reflection 1024^2: 82 us per step, 73.9 so;
+// as a called function 73.6, but the runs, which small fields wait for, slower:
+// 512^2 32.8 instead of 30.7).
+struct WallRun {
+  int corner;  // -1 interior run, else the open side (2 = W, 3 = E)
+  int m, c0;   // number of the interior run; first interior column of the lanes
+               // (even: the rows' 16-byte pairs)
+  __device__ __forceinline__ WallRun(const StageArgs& a, int b) : corner(-1), m(b) {
+    if (a.open & OPEN_W) {
+      if (m == 0) corner = 2;
+      m--;
+    }
+    if (corner < 0 && (a.open & OPEN_E)) {
+      if (m == 0) corner = 3;
+      m--;
+    }
+    c0 = corner == 2 ? BC : corner == 3 ? (a.f.nx - 2 * BC) & ~1 : BC + m * OPEN_RUN;
+  }
+};
+__device__ __forceinline__ void wall_columns(const StageArgs& a, const WallRun& run) {
+  const int lane = threadIdx.x & 31;
+  const Field& f = a.f;
+  const size_t V = f.plane, P = f.pitch;
+  const bool mw = a.mirror & NODE_W, me = a.mirror & NODE_E;
+  const int corner = run.corner, m = run.m;
+  int x = run.c0 - 1 + lane;
+  if (corner == 2 && lane == 31) x = 0;  // (lane 0 holds x = 1)
+  bool mine;
+  if (corner == 2) mine = x <= BC;
+  else if (corner == 3) mine = x >= f.nx - BC - 1 && x < f.nx;
+  else mine = lane >= (m == 0 ? 1 : 2) && lane <= 29 && x >= (mw ? BC : BC + 1) &&
+              x <= f.nx - BC - (me ? 1 : 2);
+  const double* kept = g_ring + KEEP_AT + lane;
+  double keep[5];
+#pragma unroll
+  for (int v = 0; v < 4; v++) keep[v] = kept[v * 32];
+  keep[4] = kept[ST_ROW];
+  // u^n around the first interior node
+  const int xc = min(x, f.nx - 1);
+  const double* u0 = a.u0 + 2 * P + xc;
+  WallIn in;
+  in.gr = __ldcg(u0);
+  in.gmx = __ldcg(u0 + V);
+  in.gmy = __ldcg(u0 + 2 * V);
+  in.gE = __ldcg(u0 + 3 * V);
+  in.grw = __ldcg(u0 - (xc > 0 ? 1 : 0));
+  in.gre = __ldcg(u0 + (xc < f.nx - 1 ? 1 : 0));
+  in.grs = __ldcg(u0 - P);
+  in.grn = __ldcg(u0 + P);
+  if (corner >= 0) {
+    // ghost cells of rows BC, BC+1: lanes l and 16+l hold row l of the inner
+    // and the outer layer
+    double g[4];
+    open_edge_cell<1>(a, corner, lane & 15, lane >= 16, g);
+    const int layer = corner == 2 ? 1 - x : x - (f.nx - BC);  // 0, 1 in the ghost columns
+    const int src = (layer == 1 ? 16 : 0) + BC;
+    const double g0 = __shfl_sync(0xffffffffu, g[0], src), g1 = __shfl_sync(0xffffffffu, g[1], src);
+    const double g2 = __shfl_sync(0xffffffffu, g[2], src), g3 = __shfl_sync(0xffffffffu, g[3], src);
+    const double g4 = __shfl_sync(0xffffffffu, g[0], src + 1);
+    if (layer == 0 || layer == 1) {
+      keep[0] = g0;
+      keep[1] = g1;
+      keep[2] = g2;
+      keep[3] = g3;
+      keep[4] = g4;
+    }
+  }
+  in.r1 = keep[0];
+  in.mx1 = keep[1];
+  in.my1 = keep[2];
+  in.E1 = keep[3];
+  in.r2 = keep[4];
+  in.rw = __shfl_sync(0xffffffffu, keep[0], lane - 1 & 31);  // (x = 0 is lane 31)
+  in.re = __shfl_sync(0xffffffffu, keep[0], lane + 1 & 31);
+  if (mw && x == BC) in.rw = keep[0];  // mirror image of the column itself
+  if (me && x == f.nx - BC - 1) in.re = keep[0];
+  if (!mine) return;
+  const int gt = x == 0 ? WG_L0 : (x == f.nx - 1 ? WG_R0 : WG_CENTRED);
+  unsigned int st = 0;
+  const WallOut o = wall_column(in, gt, a.xmap0 + x * a.dx, a.dx, a.dy, a.wall, a.k, &st);
+  if (st) atomicOr(a.status, st);
+  double* u = a.uout + x;
+  u[P] = o.r;
+  u[0] = o.r0;
+  u[V + P] = o.mx;
+  u[2 * V + P] = o.my;
+  // the corners of a mirror side
+  int d = 0;
+  if (mw && x < 2 * BC) d = 2 * BC - 1 - 2 * x;
+  else if (me && x >= f.nx - 2 * BC) d = 2 * (f.nx - BC) - 1 - 2 * x;
+  if (d) {
+    u[P + d] = o.r;
+    u[d] = o.r0;
+    u[V + P + d] = -o.mx;
+    u[2 * V + P + d] = o.my;
+  }
 }
 
-// grid: [ghost CTAs (OPEN only)] + strip CTAs, one warp each
-// With `join`, a dependent of the launch before it that may start while that
-// runs and must not end before it: the first CTA sees to that.
-template <int MODE, int UN, bool OPEN, bool MIX>
-__global__ void __launch_bounds__(32, WARPS) k_strip(const __grid_constant__ StageArgs a,
-                                                    int ghost_ctas, int sx, int h, int join) {
-  int b = blockIdx.x;
-  if (OPEN) {
-    if (b < ghost_ctas) {
-      if (a.node_sides) wait_for_node_pass();  // ghost frames reach the wall rows
-      open_run<MODE>(a, b);
+// What a launch does beside its strips, in its first CTAs: nothing, the
+// ghost runs of open sections, or wall runs and then ghost runs.
+enum StripEdges : int { E_NONE = 0, E_OPEN = 1, E_WALL = 2 };
+
+// CTA number b of one field (one warp per CTA): its edge_ctas edge runs, then
+// its strips, sx per band of h rows, x fastest.
+template <int MODE, int UN, int EDGES, bool MIX>
+__device__ __forceinline__ void strip_cta(const StageArgs& a, int b, int edge_ctas, int sx, int h) {
+  constexpr bool WALLS = MODE == 1 && EDGES == E_WALL;
+  bool wall = false;
+  if (EDGES && b < edge_ctas) {
+    if (WALLS) wall = b < a.wall_runs;
+    if (!wall) {
+      open_run<MODE>(a, b - (WALLS ? a.wall_runs : 0));
       return;
     }
-    b -= ghost_ctas;
+  } else {
+    b -= edge_ctas;
   }
-  strip_cta<MODE, UN, MIX>(a, b, sx, h);
-  if (!OPEN && join && blockIdx.x == 0) wait_for_node_pass();
+  // MODE 2 (buffer-layer grid): strips over the border box, the first one
+  // starting at an even column so that the rows' 16-byte pairs stay aligned
+  int c0 = (MODE == 2 ? (a.box_x0 & ~1) : BC) + (b % sx) * SW;
+  int y0 = (MODE == 2 ? a.box_y0 : BC) + (b / sx) * h;
+  const int ylast = MODE == 2 ? a.box_y1 : a.f.ny - BC - 1;
+  int y1 = min(y0 + h, ylast + 1);
+  if (WALLS) {
+    const WallRun run(a, b);
+    if (wall) {
+      c0 = run.c0;
+      y0 = BC;
+      y1 = BC + 2;
+    }
+    strip_warp<MODE, UN, MIX, true>(a, c0, y0, y1, wall);
+    if (wall) wall_columns(a, run);
+  } else {
+    strip_warp<MODE, UN, MIX>(a, c0, y0, y1);
+  }
+}
+
+template <int MODE, int UN, int EDGES, bool MIX>
+__global__ void __launch_bounds__(32, WARPS) k_strip(const __grid_constant__ StageArgs a,
+                                                    int edge_ctas, int sx, int h) {
+  strip_cta<MODE, UN, EDGES, MIX>(a, blockIdx.x, edge_ctas, sx, h);
+  if (EDGES == E_NONE && a.apart && blockIdx.x == 0) wait_for_launch_before();
 }
 
 // the ghost runs alone (open_runs_apart)
 template <int MODE>
 __global__ void __launch_bounds__(32) k_open_runs(const __grid_constant__ StageArgs a) {
-  asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+  wait_for_launch_before();
+  let_dependents_start();
   open_run<MODE>(a, blockIdx.x);
 }
 
@@ -831,7 +992,10 @@ __device__ __forceinline__ StageArgs batch_stage_args(const BatchStageArgs& P, i
   a.wall_s = d.wall_s;
   a.variant = 0;
   a.open = d.open;
-  a.node_sides = d.node_sides;
+  a.mirror = d.mirror;
+  a.wall_runs = d.wall_runs;
+  a.status = d.status;
+  a.apart = 0;
   a.mixed = 0;
   a.t = 0.0;
   a.xmap0 = d.xmap0;
@@ -843,39 +1007,33 @@ __device__ __forceinline__ StageArgs batch_stage_args(const BatchStageArgs& P, i
   return a;
 }
 
-// last domain i in [0, n) whose first CTA (ghost0 or strip0) is <= b
-template <bool GHOST>
+// last domain i in [0, n) whose first CTA (edge0 or strip0) is <= b
+template <bool EDGES>
 __device__ __forceinline__ int batch_domain(const BatchStageArgs& P, int b) {
   int lo = 0, hi = P.ndom - 1;
   while (lo < hi) {
     const int mid = (lo + hi + 1) >> 1;
-    const int first = GHOST ? P.d[mid].ghost0 : P.d[mid].strip0;
+    const int first = EDGES ? P.d[mid].edge0 : P.d[mid].strip0;
     if (first <= b) lo = mid;
     else hi = mid - 1;
   }
   return lo;
 }
 
-// One RK stage of every domain of a batch (one boundary kind): the ghost
-// CTAs of all domains first (open and wall kinds: each domain's open
-// sections), then every domain's strip CTAs.
-template <int UN, bool OPEN, bool MIX>
+// One RK stage of every domain of a batch (one boundary kind): the edge runs of
+// all domains first, then every domain's strips.
+template <int UN, int EDGES, bool MIX>
 __global__ void __launch_bounds__(32, WARPS)
     k_strip_batch(const __grid_constant__ BatchStageArgs P, int h) {
   int b = blockIdx.x;
-  if (OPEN) {
-    if (b < P.ghost_ctas) {
-      const int i = batch_domain<true>(P, b);
-      const StageArgs a = batch_stage_args<false>(P, i);
-      if (a.node_sides) wait_for_node_pass();
-      open_run<1>(a, b - P.d[i].ghost0);
-      return;
-    }
-    b -= P.ghost_ctas;
-  }
-  const int i = batch_domain<false>(P, b);
+  const bool edge = EDGES && b < P.edge_ctas;
+  if (!edge) b -= P.edge_ctas;
+  const int i = edge ? batch_domain<true>(P, b) : batch_domain<false>(P, b);
   const StageArgs a = batch_stage_args<MIX>(P, i);
-  strip_cta<1, UN, MIX>(a, b - P.d[i].strip0, P.d[i].sx, h);
+  const BatchDomain& d = P.d[i];
+  // its edge runs are numbered from 0, its strips from edge_ctas
+  strip_cta<1, UN, EDGES, MIX>(a, edge ? b - d.edge0 : P.edge_ctas + b - d.strip0, P.edge_ctas,
+                               d.sx, h);
 }
 
 // ---- persistent batched kernel -----------------------------------------
@@ -952,7 +1110,9 @@ __device__ __forceinline__ StageArgs persist_stage_args(const PersistArgs& P, co
   a.t = 0.0;
   a.xmap0 = d.xmap0;
   a.ymap0 = d.ymap0;
-  a.node_sides = 0;  // the item order already waits for the node pass
+  a.mirror = a.wall_runs = 0;  // its items
+  a.status = nullptr;
+  a.apart = 0;
   a.mask = nullptr;
   a.box_x0 = a.box_x1 = a.box_y0 = a.box_y1 = 0;
   a.wall = P.wall;
@@ -1080,25 +1240,12 @@ __global__ void __launch_bounds__(32 * PW, 8) k_batch_persistent(const __grid_co
   }
 }
 
-// launch of one-warp CTAs; with `after_node_pass`, as a programmatic
-// dependent of the node pass launched just before on `s` (it may start while
-// the pass runs)
-inline cudaError_t launch_after_node_pass(const void* fn, unsigned blocks, cudaStream_t s,
-                                          bool after_node_pass, void** args) {
+// launch of one-warp CTAs with their rings
+inline cudaError_t launch_strips(const void* fn, unsigned blocks, cudaStream_t s, void** args) {
   cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout,
                                        cudaSharedmemCarveoutMaxShared);
   if (e != cudaSuccess) return e;
-  cudaLaunchConfig_t cfg = {};
-  cfg.dynamicSmemBytes = WARP_DOUBLES * sizeof(double);
-  cfg.gridDim = dim3(blocks);
-  cfg.blockDim = dim3(32);
-  cfg.stream = s;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = after_node_pass ? 1 : 0;
-  return cudaLaunchKernelExC(&cfg, fn, args);
+  return launch_dependent(fn, blocks, 32, WARP_DOUBLES * sizeof(double), s, args);
 }
 
 // rows per strip of shape 0..4
@@ -1122,24 +1269,27 @@ int rows_of(int shape, Strips strips) {
   while (h < 16 && strips(h) > 148LL * WARPS) h *= 2;
   return h;
 }
-template <int MODE, int UN, bool MIX>
-const void* strip_fn(bool open) {
-  return open ? (const void*)k_strip<MODE, UN, true, MIX>
-              : (const void*)k_strip<MODE, UN, false, MIX>;
+template <int UN, bool MIX>
+const void* stage_fn(int edges) {
+  return edges == E_WALL   ? (const void*)k_strip<1, UN, E_WALL, MIX>
+         : edges == E_OPEN ? (const void*)k_strip<1, UN, E_OPEN, MIX>
+                           : (const void*)k_strip<1, UN, E_NONE, MIX>;
 }
-const void* strip_fn(int mode, bool un, bool open, bool mixed) {
-  if (mode == 0) return mixed ? strip_fn<0, 0, true>(open) : strip_fn<0, 0, false>(open);
-  if (un) return mixed ? strip_fn<1, 1, true>(open) : strip_fn<1, 1, false>(open);
-  return mixed ? strip_fn<1, 0, true>(open) : strip_fn<1, 0, false>(open);
+template <bool MIX>
+const void* strip_fn(int mode, bool un, int edges) {
+  if (mode == 0)
+    return edges ? (const void*)k_strip<0, 0, E_OPEN, MIX> : (const void*)k_strip<0, 0, E_NONE, MIX>;
+  return un ? stage_fn<1, MIX>(edges) : stage_fn<0, MIX>(edges);
 }
 
 int strips_across(const Field& f) { return (f.nx - 2 * BC + SW - 1) / SW; }
 int strips_up(const Field& f, int h) { return (f.ny - 2 * BC + h - 1) / h; }
 
 template <int UN, bool MIX>
-const void* strip_batch_fn(bool open) {
-  return open ? (const void*)k_strip_batch<UN, true, MIX>
-              : (const void*)k_strip_batch<UN, false, MIX>;
+const void* strip_batch_fn(int kind) {
+  return kind == BK_WALL   ? (const void*)k_strip_batch<UN, E_WALL, MIX>
+         : kind == BK_OPEN ? (const void*)k_strip_batch<UN, E_OPEN, MIX>
+                           : (const void*)k_strip_batch<UN, E_NONE, MIX>;
 }
 
 }  // namespace
@@ -1172,24 +1322,21 @@ cudaError_t launch_strip_batch(BatchStageArgs& P, int kind, int shape, bool mixe
       n += (long long)strips_across(P.d[i].f) * strips_up(P.d[i].f, rows);
     return n;
   });
-  const bool open = kind == BK_OPEN || kind == BK_WALL;
   long long ghost = 0, strips = 0;
-  bool pdl = false;
   for (int i = 0; i < P.ndom; i++) {
     BatchDomain& d = P.d[i];
     d.sx = strips_across(d.f);
-    d.ghost0 = (int)ghost;
+    d.edge0 = (int)ghost;
     d.strip0 = (int)strips;
-    if (open) ghost += open_run_count(d.f, d.open);
+    if (kind != BK_PLAIN) ghost += d.wall_runs + open_run_count(d.f, d.open);
     strips += (long long)d.sx * strips_up(d.f, h);
-    pdl = pdl || d.node_sides != 0;
   }
   if (ghost + strips > 0x7fffffffLL) return cudaErrorInvalidValue;
-  P.ghost_ctas = (int)ghost;
-  const void* fn = P.stage != 1 ? (mixed ? strip_batch_fn<1, true>(open) : strip_batch_fn<1, false>(open))
-                                : (mixed ? strip_batch_fn<0, true>(open) : strip_batch_fn<0, false>(open));
+  P.edge_ctas = (int)ghost;
+  const void* fn = P.stage != 1 ? (mixed ? strip_batch_fn<1, true>(kind) : strip_batch_fn<1, false>(kind))
+                                : (mixed ? strip_batch_fn<0, true>(kind) : strip_batch_fn<0, false>(kind));
   void* args[] = {&P, &h};
-  return launch_after_node_pass(fn, (unsigned)(ghost + strips), s, pdl, args);
+  return launch_strips(fn, (unsigned)(ghost + strips), s, args);
 }
 
 // L(u) of a buffer-layer grid at its interior_pt points (MODE 2) over the
@@ -1199,32 +1346,34 @@ cudaError_t launch_strip_masked(const StageArgs& a, cudaStream_t s) {
   int sx = (a.box_x1 - (a.box_x0 & ~1) + SW) / SW;
   const int rows = a.box_y1 - a.box_y0 + 1;
   int h = rows_of(SHAPE_BY_SIZE, [&](int r) { return (long long)sx * ((rows + r - 1) / r); });
-  int ghost_ctas = 0, join = 0;
+  int edge_ctas = 0;
   StageArgs aa = a;
-  void* args[] = {&aa, &ghost_ctas, &sx, &h, &join};
-  return launch_after_node_pass(strip_fn<2, 0, false>(false), (unsigned)sx * (unsigned)((rows + h - 1) / h), s,
-                                false, args);
+  void* args[] = {&aa, &edge_ctas, &sx, &h};
+  return launch_strips((const void*)k_strip<2, 0, E_NONE, false>,
+                       (unsigned)sx * (unsigned)((rows + h - 1) / h), s, args);
 }
 
 cudaError_t launch_strip_stage(const StageArgs& a, int mode, int shape, cudaStream_t s) {
   if (shape < SHAPE_BY_SIZE || shape > 4) return cudaErrorInvalidValue;
   int sx = strips_across(a.f);
   int h = rows_of(shape, [&](int rows) { return (long long)sx * strips_up(a.f, rows); });
-  int join = open_runs_apart(a);
-  int ghost_ctas = join ? 0 : open_run_count(a.f, a.open);
-  const bool open = ghost_ctas > 0;
-  const void* fn = strip_fn(mode, a.stage != 1, open, a.mixed);
+  const int walls = mode == 1 ? a.wall_runs : 0;
+  int edge_ctas = walls + (a.apart ? 0 : open_run_count(a.f, a.open));
+  const int edges = walls ? E_WALL : (edge_ctas ? E_OPEN : E_NONE);
+  const void* fn = a.mixed ? strip_fn<true>(mode, a.stage != 1, edges)
+                           : strip_fn<false>(mode, a.stage != 1, edges);
   StageArgs aa = a;
-  void* args[] = {&aa, &ghost_ctas, &sx, &h, &join};
-  return launch_after_node_pass(fn, (unsigned)ghost_ctas + (unsigned)sx * (unsigned)strips_up(a.f, h),
-                                s, a.node_sides != 0 || join, args);
+  void* args[] = {&aa, &edge_ctas, &sx, &h};
+  return launch_strips(fn, (unsigned)edge_ctas + (unsigned)sx * (unsigned)strips_up(a.f, h), s,
+                       args);
 }
 
 cudaError_t launch_open_runs(const StageArgs& a, int mode, cudaStream_t s) {
   const unsigned n = (unsigned)open_run_count(a.f, a.open);
-  if (mode == 0) k_open_runs<0><<<n, 32, 0, s>>>(a);
-  else k_open_runs<1><<<n, 32, 0, s>>>(a);
-  return cudaGetLastError();
+  StageArgs aa = a;
+  void* args[] = {&aa};
+  return launch_dependent(mode == 0 ? (const void*)k_open_runs<0> : (const void*)k_open_runs<1>, n,
+                          32, 0, s, args);
 }
 
 }  // namespace dim2d
