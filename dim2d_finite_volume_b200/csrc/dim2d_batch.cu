@@ -14,7 +14,7 @@
 // One RK stage of a group is one batched launch over all its domains, so a
 // step is at most 8 x 3 launches however many domains there are.  The groups are independent: a captured step
 // graph holds one chain per group as parallel branches, so the kinds
-// overlap on the device.  Two graphs are kept, one per buffer parity
+// overlap on the device.  Graphs of several steps are kept by buffer parity
 // (which of A/B holds u^n), and rebuilt when members, dt or shapes change.
 #include <algorithm>
 #include <cmath>
@@ -23,8 +23,6 @@
 #include <vector>
 
 #include "dim2d_internal.h"
-#include "dim2d_nodebc.cuh"
-#include "dim2d_open.cuh"
 
 using namespace dim2d;
 
@@ -56,9 +54,8 @@ struct dim2d_batch {
   dim2d_params p{};
   int shape[NGROUPS];  // strip shape of each group, SHAPE_BY_SIZE until set or tuned
   bool use_graphs = true;
-  cudaGraphExec_t graph[2] = {nullptr, nullptr};
-  long long graph_launches[2] = {0, 0};
-  bool graphs_valid = false;
+  // by size and parity of the steps since they were dropped
+  StepGraph graph[GRAPH_SIZES][2];
   int parity = 0;
   long long launches = 0;
   // persistent mode (dim2d_batch_set_persistent): one kernel per precision
@@ -74,19 +71,20 @@ struct dim2d_batch {
 namespace {
 
 void drop_batch_graphs(dim2d_batch* b) {
-  for (int i = 0; i < 2; i++) {
-    if (b->graph[i]) cudaGraphExecDestroy(b->graph[i]);
-    b->graph[i] = nullptr;
-  }
-  b->graphs_valid = false;
+  for (auto& size : b->graph)
+    for (StepGraph& g : size) {
+      if (g.exec) cudaGraphExecDestroy(g.exec);
+      g = StepGraph();
+    }
   b->parity = 0;
 }
 
 // Stage `st` of the members of group g (indices idx), one batched launch per
 // BATCH_MAX of them.  in/out per stage: 1: A->B, 2: B->C, 3: C->B,
-// u^n = A.  dt_scale 0 gives the dry step of the autotuner.
+// u^n = A; A and B change places in odd steps.  dt_scale 0 gives the dry step
+// of the autotuner.
 cudaError_t group_stage(dim2d_batch* b, int g, const std::vector<int>& idx, int st, int shape,
-                        double dt_scale, cudaStream_t s) {
+                        double dt_scale, cudaStream_t s, bool odd = false) {
   static thread_local BatchStageArgs P;
   for (size_t c0 = 0; c0 < idx.size(); c0 += BATCH_MAX) {
     const int n = (int)std::min<size_t>(BATCH_MAX, idx.size() - c0);
@@ -99,12 +97,14 @@ cudaError_t group_stage(dim2d_batch* b, int g, const std::vector<int>& idx, int 
     for (int j = 0; j < n; j++) {
       const int i = idx[c0 + j];
       dim2d_handle* h = b->m[i];
-      const double* in = st == 1 ? h->A : (st == 2 ? h->B : h->C);
-      double* out = st == 2 ? h->C : h->B;
+      double* const A = odd ? h->B : h->A;
+      double* const B = odd ? h->A : h->B;
+      const double* in = st == 1 ? A : (st == 2 ? B : h->C);
+      double* out = st == 2 ? h->C : B;
       BatchDomain& d = P.d[j];
       d.f = h->f;
       d.uin = in;
-      d.u0 = h->A;
+      d.u0 = A;
       d.uout = out;
       d.dx = h->dx;
       d.dy = h->dy;
@@ -134,16 +134,17 @@ std::vector<int> members_of(const dim2d_batch* b, int g) {
   return idx;
 }
 
-// One step of every group, each group's chain on its own stream forked from
-// b->stream (so the chains overlap); joined back into b->stream.
-cudaError_t launch_step(dim2d_batch* b, double dt_scale) {
+// `steps` steps of every group, each group's chain on its own stream forked
+// from b->stream (so the chains overlap, and one group need not wait for
+// another between its steps); joined back into b->stream.
+cudaError_t launch_steps(dim2d_batch* b, int steps) {
   cudaError_t e = cudaEventRecord(b->fork, b->stream);
   for (int g = 0; g < NGROUPS && e == cudaSuccess; g++) {
     const std::vector<int> idx = members_of(b, g);
     if (idx.empty()) continue;
     e = cudaStreamWaitEvent(b->side[g], b->fork, 0);
-    for (int st = 1; st <= 3 && e == cudaSuccess; st++)
-      e = group_stage(b, g, idx, st, b->shape[g], dt_scale, b->side[g]);
+    for (int k = 0; k < 3 * steps && e == cudaSuccess; k++)
+      e = group_stage(b, g, idx, k % 3 + 1, b->shape[g], 1.0, b->side[g], k / 3 & 1);
     if (e == cudaSuccess) e = cudaEventRecord(b->join[g], b->side[g]);
     if (e == cudaSuccess) e = cudaStreamWaitEvent(b->stream, b->join[g], 0);
   }
@@ -154,44 +155,27 @@ void swap_members(dim2d_batch* b) {
   for (dim2d_handle* h : b->m) std::swap(h->A, h->B);
 }
 
-// capture the step graph of the current buffer parity into slot `slot`
-int capture(dim2d_batch* b, int slot) {
+// capture `steps` steps from the current buffer parity into g
+int capture(dim2d_batch* b, StepGraph& g, int steps) {
   const long long n0 = b->launches;
   cudaError_t e = cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeRelaxed);
   if (e != cudaSuccess) {
     cudaGetLastError();
     return DIM2D_ERR_UNSUPPORTED;
   }
-  cudaError_t el = launch_step(b, 1.0);
-  cudaGraph_t g = nullptr;
-  e = cudaStreamEndCapture(b->stream, &g);
-  b->graph_launches[slot] = b->launches - n0;
+  cudaError_t el = launch_steps(b, steps);
+  cudaGraph_t graph = nullptr;
+  e = cudaStreamEndCapture(b->stream, &graph);
+  g.launches = b->launches - n0;
   b->launches = n0;
   cudaGraphExec_t x = nullptr;
-  if (el == cudaSuccess && e == cudaSuccess && g) e = cudaGraphInstantiate(&x, g, 0);
-  if (g) cudaGraphDestroy(g);
+  if (el == cudaSuccess && e == cudaSuccess && graph) e = cudaGraphInstantiate(&x, graph, 0);
+  if (graph) cudaGraphDestroy(graph);
   if (el != cudaSuccess || e != cudaSuccess || !x) {
     cudaGetLastError();
     return el != cudaSuccess ? cuda_error(el, "batch capture") : DIM2D_ERR_UNSUPPORTED;
   }
-  b->graph[slot] = x;
-  return DIM2D_OK;
-}
-
-int build_graphs(dim2d_batch* b) {
-  drop_batch_graphs(b);
-  int rc = capture(b, 0);
-  if (!rc) {
-    swap_members(b);  // host view of the other parity; nothing runs
-    rc = capture(b, 1);
-    swap_members(b);
-  }
-  if (rc) {
-    drop_batch_graphs(b);
-    return rc;
-  }
-  b->graphs_valid = true;
-  b->parity = 0;
+  g.exec = x;
   return DIM2D_OK;
 }
 
@@ -416,24 +400,33 @@ int dim2d_batch_step(dim2d_batch* b, int nsteps) {
       for (int k = 0; k < nsteps; k++) b->m[i]->t += b->dt[i];
     return publish(b);
   }
-  if (b->use_graphs && !b->graphs_valid) {
-    int rc = build_graphs(b);
-    if (rc && rc != DIM2D_ERR_UNSUPPORTED) return rc;
-  }
-  for (int s = 0; s < nsteps; s++) {
-    if (b->use_graphs && b->graphs_valid) {
-      cudaError_t e = cudaGraphLaunch(b->graph[b->parity], b->stream);
-      if (e != cudaSuccess) return cuda_error(e, "batch step graph");
-      b->launches += b->graph_launches[b->parity];
-      b->parity ^= 1;
-    } else {
-      cudaError_t e = launch_step(b, 1.0);
-      if (e != cudaSuccess) return cuda_error(e, "batch step");
-      // the two graphs follow the buffer parity; a stream step flips it too
-      b->parity ^= 1;
+  for (int s = 0; s < nsteps;) {
+    const int size = graph_size_for(nsteps - s);
+    int n = GRAPH_STEPS[size];
+    StepGraph* g = nullptr;
+    if (b->use_graphs) {
+      g = &b->graph[size][b->parity];
+      if (!g->exec) {
+        int rc = capture(b, *g, n);
+        if (rc && rc != DIM2D_ERR_UNSUPPORTED) return rc;
+      }
     }
-    swap_members(b);  // the host side of rk3_step for every member
-    for (size_t i = 0; i < b->m.size(); i++) b->m[i]->t += b->dt[i];  // field_class.f:70
+    if (g && g->exec) {
+      cudaError_t e = cudaGraphLaunch(g->exec, b->stream);
+      if (e != cudaSuccess) return cuda_error(e, "batch step graph");
+      b->launches += g->launches;
+    } else {
+      n = 1;
+      cudaError_t e = launch_steps(b, n);
+      if (e != cudaSuccess) return cuda_error(e, "batch step");
+    }
+    // the graphs follow the buffer parity, and so do steps without them
+    b->parity ^= n & 1;
+    for (int k = 0; k < n; k++) {
+      swap_members(b);  // the host side of rk3_step for every member
+      for (size_t i = 0; i < b->m.size(); i++) b->m[i]->t += b->dt[i];  // field_class.f:70
+    }
+    s += n;
   }
   return publish(b);
 }

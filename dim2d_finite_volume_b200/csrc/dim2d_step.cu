@@ -168,22 +168,20 @@ cudaError_t wait_copy_if(dim2d_handle* h, const double* target) {
 }
 
 void drop_graphs(dim2d_handle* h) {
-  for (int i = 0; i < 2; i++) {
-    if (h->graph_exec[i]) cudaGraphExecDestroy(h->graph_exec[i]);
-    h->graph_exec[i] = nullptr;
-    h->graph_A[i] = nullptr;
-  }
+  for (auto& size : h->graph)
+    for (StepGraph& g : size) {
+      if (g.exec) cudaGraphExecDestroy(g.exec);
+      g = StepGraph();
+    }
 }
 
-// Capture one RK3 step into graph slot `slot`.  The capture runs
-// rk3_step's host side (A/B swap, time += dt) without executing anything;
-// on success the caller launches the graph once, which brings the device
-// state to the host state.  On failure the host side is rolled back.  No
+// Capture `steps` RK3 steps into sg.  The capture runs
+// rk3_step's host side (A/B swap, time += dt) without executing anything; it
+// is rolled back, and the caller applies it per launch (replayed).  No
 // kernel reads the field time, so one graph serves every time level.
-static int capture_step(dim2d_handle* h, double dt, int slot) {
-  if (h->graph_exec[slot]) cudaGraphExecDestroy(h->graph_exec[slot]);
-  h->graph_exec[slot] = nullptr;
-  h->graph_A[slot] = nullptr;
+static int capture_steps(dim2d_handle* h, double dt, StepGraph& sg, int steps) {
+  if (sg.exec) cudaGraphExecDestroy(sg.exec);
+  sg = StepGraph();
   double* const A0 = h->A;
   double* const B0 = h->B;
   const double t0 = h->t;
@@ -193,24 +191,24 @@ static int capture_step(dim2d_handle* h, double dt, int slot) {
     cudaGetLastError();
     return DIM2D_ERR_UNSUPPORTED;  // e.g. the legacy default stream
   }
-  const int rc = rk3_step(h, dt);
+  int rc = DIM2D_OK;
+  for (int s = 0; s < steps && !rc; s++) rc = rk3_step(h, dt);
   cudaGraph_t g = nullptr;
   e = cudaStreamEndCapture(h->stream, &g);
-  const long long n = h->launches - n0;
+  sg.launches = h->launches - n0;
   h->launches = n0;
+  h->A = A0;
+  h->B = B0;
+  h->t = t0;
   cudaGraphExec_t x = nullptr;
   if (!rc && e == cudaSuccess && g) e = cudaGraphInstantiate(&x, g, 0);
   if (g) cudaGraphDestroy(g);
   if (rc || e != cudaSuccess || !x) {
     cudaGetLastError();
-    h->A = A0;
-    h->B = B0;
-    h->t = t0;
     return rc ? rc : DIM2D_ERR_UNSUPPORTED;
   }
-  h->graph_exec[slot] = x;
-  h->graph_A[slot] = A0;
-  h->graph_launches[slot] = n;
+  sg.exec = x;
+  sg.A = A0;
   return DIM2D_OK;
 }
 
@@ -270,33 +268,38 @@ int rk3_steps(dim2d_handle* h, double dt, int nsteps) {
     drop_graphs(h);
     h->graph_dt = dt;
   }
-  for (int s = 0; s < nsteps; s++) {
-    // stage 1 writes B: a pending asynchronous copy of B must land first
+  for (int s = 0; s < nsteps;) {
+    // stage 1 writes B (and, a step on, A): pending asynchronous copies of
+    // them must land first
+    const int size = graph_size_for(nsteps - s);
+    const int n = graphs ? GRAPH_STEPS[size] : 1;
     cudaError_t ew = wait_copy_if(h, h->B);
+    if (ew == cudaSuccess && n > 1) ew = wait_copy_if(h, h->A);
     if (ew != cudaSuccess) return cuda_error(ew, "step");
     if (graphs) {
-      int slot = -1;
+      StepGraph* const slots = h->graph[size];
+      StepGraph* g = nullptr;
       for (int i = 0; i < 2; i++)
-        if (h->graph_exec[i] && h->graph_A[i] == h->A) slot = i;
-      bool fresh = false;
-      if (slot < 0) {
-        slot = (h->graph_exec[0] && h->graph_A[0] != h->A) ? 1 : 0;
-        fresh = capture_step(h, dt, slot) == DIM2D_OK;
-        if (!fresh) slot = -1;
+        if (slots[i].exec && slots[i].A == h->A) g = &slots[i];
+      if (!g) {
+        StepGraph& free = slots[slots[0].exec && slots[0].A != h->A ? 1 : 0];
+        if (capture_steps(h, dt, free, n) == DIM2D_OK) g = &free;
       }
-      if (slot >= 0) {
-        cudaError_t e = cudaGraphLaunch(h->graph_exec[slot], h->stream);
+      if (g) {
+        cudaError_t e = cudaGraphLaunch(g->exec, h->stream);
         if (e != cudaSuccess) return cuda_error(e, "step graph");
-        h->launches += h->graph_launches[slot];
-        if (!fresh) {  // the host side of rk3_step
+        h->launches += g->launches;
+        for (int i = 0; i < n; i++) {  // the host side of rk3_step
           std::swap(h->A, h->B);
           h->t += dt;  // field_class.f:70
         }
+        s += n;
         continue;
       }
     }
     int rc = rk3_step(h, dt);
     if (rc) return rc;
+    s++;
   }
   return DIM2D_OK;
 }
