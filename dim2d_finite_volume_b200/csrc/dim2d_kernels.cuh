@@ -128,6 +128,12 @@ struct StageArgs {
   int wall_runs;                       // south wall: runs of wall columns whose ghost cells
                                        // the launch solves (wall_run_count)
   unsigned int* status;                // wall root status word
+  int reverse;                         // strips from the last to the first: every other
+                                       // launch of a run, so that a stage starts on the
+                                       // rows that the one before left in L2 (sustained,
+                                       // us per step: 2048^2 open 269 -> 260, mixed wall
+                                       // 256 -> 249; evicting dead inputs first: no gain;
+                                       // batches, whose kinds overlap: 1 % slower, never)
   int apart;                           // its ghost cells take the launch before (open_runs_apart)
   const int* __restrict__ mask;        // time derivative of a buffer-layer grid: its
                                        // grdpts_id map, written only where it is

@@ -34,6 +34,8 @@ StageArgs make_stage_args(const dim2d_handle* h, const double* uin, double* uout
   a.t = h->t;
   a.xmap0 = h->xmap0;
   a.ymap0 = h->ymap0;
+  // every other launch of a run of steps (A and B change places each step)
+  a.reverse = (st & 1) ^ (h->A < h->B);
   a.mirror = h->mirror_sides;
   a.wall_runs = h->south_wall ? wall_run_count(h->f, h->open_mask) : 0;
   a.status = h->status;

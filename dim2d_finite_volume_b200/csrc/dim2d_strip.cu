@@ -960,7 +960,9 @@ __device__ __forceinline__ void strip_cta(const StageArgs& a, int b, int edge_ct
 template <int MODE, int UN, int EDGES, bool MIX>
 __global__ void __launch_bounds__(32, WARPS) k_strip(const __grid_constant__ StageArgs a,
                                                     int edge_ctas, int sx, int h) {
-  strip_cta<MODE, UN, EDGES, MIX>(a, blockIdx.x, edge_ctas, sx, h);
+  int b = blockIdx.x;
+  if (a.reverse && b >= edge_ctas) b = edge_ctas + (int)gridDim.x - 1 - b;
+  strip_cta<MODE, UN, EDGES, MIX>(a, b, edge_ctas, sx, h);
   if (EDGES == E_NONE && a.apart && blockIdx.x == 0) wait_for_launch_before();
 }
 
@@ -995,7 +997,7 @@ __device__ __forceinline__ StageArgs batch_stage_args(const BatchStageArgs& P, i
   a.mirror = d.mirror;
   a.wall_runs = d.wall_runs;
   a.status = d.status;
-  a.apart = 0;
+  a.apart = a.reverse = 0;
   a.mixed = 0;
   a.t = 0.0;
   a.xmap0 = d.xmap0;
@@ -1112,7 +1114,7 @@ __device__ __forceinline__ StageArgs persist_stage_args(const PersistArgs& P, co
   a.ymap0 = d.ymap0;
   a.mirror = a.wall_runs = 0;  // its items
   a.status = nullptr;
-  a.apart = 0;
+  a.apart = a.reverse = 0;
   a.mask = nullptr;
   a.box_x0 = a.box_x1 = a.box_y0 = a.box_y1 = 0;
   a.wall = P.wall;
