@@ -155,11 +155,11 @@ __device__ __forceinline__ void wait_for_launch_before() {
   asm volatile("griddepcontrol.wait;\n" ::: "memory");
 }
 // launch as a programmatic dependent of the launch before it on `s`
-inline cudaError_t launch_dependent(const void* fn, unsigned blocks, unsigned threads, size_t smem,
+inline cudaError_t launch_dependent(const void* fn, dim3 blocks, dim3 threads, size_t smem,
                                     cudaStream_t s, void** args) {
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(blocks);
-  cfg.blockDim = dim3(threads);
+  cfg.gridDim = blocks;
+  cfg.blockDim = threads;
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
   cudaLaunchAttribute attr[1];
