@@ -36,16 +36,10 @@ constexpr int SM_FX = 4 * TY * (TX + 1);
 constexpr int SM_FY = 4 * (TY + 1) * TX;
 constexpr int SM_DOUBLES = SM_RAW + SM_PRIM + SM_FX + SM_FY;
 
-// Caller-provided layouts that the strip kernels cannot read (odd nx or
-// misaligned planes).  Mode 1 = RK stage update (periodic or open field),
-// 2 = L(u) of a buffer-layer grid: tiles over [box_x0, box_x1] x
-// [box_y0, box_y1], written where the grdpts_id map is interior_pt.  A face
-// whose stencil reaches a no_pt node (whatever it holds) feeds only points
-// that are not interior_pt: every point within two of an interior_pt point is
-// a boundary point of the layer.
+// The RK stage of caller-provided layouts that the strip kernels cannot read
+// (odd nx or misaligned planes; periodic or open field).
 // Four 256-thread CTAs per SM (64 registers, no spills; 4 x 47.8 KB of shared
 // memory): with three, the face pass left the FP64 pipe waiting on latency.
-template <int MODE>
 __global__ void __launch_bounds__(NT, 4) k_interior(StageArgs a) {
   extern __shared__ __align__(16) double sm[];
   double* sR = sm;
@@ -62,8 +56,8 @@ __global__ void __launch_bounds__(NT, 4) k_interior(StageArgs a) {
   double* sFy = sFx + SM_FX;
 
   const Field f = a.f;
-  const int x0 = (MODE == 2 ? a.box_x0 : BC) + blockIdx.x * TX;
-  const int y0 = (MODE == 2 ? a.box_y0 : BC) + blockIdx.y * TY;
+  const int x0 = BC + blockIdx.x * TX;
+  const int y0 = BC + blockIdx.y * TY;
   const int tid = threadIdx.x;
 
   // 1. halo tile of the input state (rows are contiguous in HBM)
@@ -186,7 +180,6 @@ __global__ void __launch_bounds__(NT, 4) k_interior(StageArgs a) {
   const int o = (ty + 2) * LX + tx + 2;
   const double uc[4] = {sR[o], sMx[o], sMy[o], sE[o]};
   const size_t go = (size_t)gy * f.pitch + gx;
-  if (MODE == 2 && (gx > a.box_x1 || gy > a.box_y1 || __ldg(a.mask + go) != 1)) return;
   // periodic images of this cell in the ghost layers
   int ix2 = -1, iy2 = -1;
   if (a.periodic) {
@@ -207,9 +200,7 @@ __global__ void __launch_bounds__(NT, 4) k_interior(StageArgs a) {
       if (v == 3) L += -uc[2] * k.gravity;
     }
     double out;
-    if (MODE != 1) {
-      out = L;
-    } else if (a.stage == 1) {
+    if (a.stage == 1) {
       out = uc[v] + a.dt * L;
     } else {
       const double u0 = __ldg(a.u0 + go + v * f.plane);
@@ -217,7 +208,7 @@ __global__ void __launch_bounds__(NT, 4) k_interior(StageArgs a) {
     }
     double* dst = a.uout + v * f.plane;
     dst[go] = out;
-    if (MODE == 1 && a.periodic) {
+    if (a.periodic) {
       if (ix2 >= 0) dst[(size_t)gy * f.pitch + ix2] = out;
       if (iy2 >= 0) {
         dst[(size_t)iy2 * f.pitch + gx] = out;
@@ -285,8 +276,8 @@ static cudaError_t set_smem_attr() {
   if (e != cudaSuccess) return e;
   if (dev >= 0 && dev < 64 && done[dev]) return cudaSuccess;
   const int bytes = (int)interior_smem_bytes();
-  const void* fns[2] = {(const void*)k_interior<1>, (const void*)k_interior<2>};
-  for (const void* fn : fns) {
+  const void* fn = (const void*)k_interior;
+  {
     e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     if (e != cudaSuccess) return e;
     // four resident CTAs need the largest shared-memory carveout
@@ -304,22 +295,13 @@ cudaError_t launch_interior_stage(const StageArgs& a, cudaStream_t s) {
   cudaError_t e = set_smem_attr();
   if (e != cudaSuccess) return e;
   dim3 grid((a.f.nx - 2 * BC + TX - 1) / TX, (a.f.ny - 2 * BC + TY - 1) / TY);
-  k_interior<1><<<grid, NT, interior_smem_bytes(), s>>>(a);
+  k_interior<<<grid, NT, interior_smem_bytes(), s>>>(a);
   return cudaGetLastError();
 }
 
 // of a field that the library allocated: its layout suits the strips
 cudaError_t launch_time_dev(const StageArgs& a, cudaStream_t s) {
   return launch_strip_stage(a, 0, strip_shape_of(a), s);
-}
-
-cudaError_t launch_time_dev_masked(const StageArgs& a, cudaStream_t s) {
-  if (strip_layout_ok(a)) return launch_strip_masked(a, s);
-  cudaError_t e = set_smem_attr();
-  if (e != cudaSuccess) return e;
-  dim3 grid((a.box_x1 - a.box_x0 + TX) / TX, (a.box_y1 - a.box_y0 + TY) / TY);
-  k_interior<2><<<grid, NT, interior_smem_bytes(), s>>>(a);
-  return cudaGetLastError();
 }
 
 cudaError_t launch_fill(double* p, double v, size_t n, cudaStream_t s) {

@@ -7,10 +7,8 @@
 // (3) (parameters_bf_layer.f:41-44).  These kernels are the area-sized part
 // of stepping such a grid:
 //   * time derivative at the interior_pt points inside the borders
-//     (td_operators_class.f:293-417): the warp-strip kernel (k_strip,
-//     dim2d_strip.cu) where nx is even and the nodes 16-byte aligned, else
-//     the interior tile kernel (k_interior, dim2d_interior.cu), over the
-//     border box, in their masked mode -- primitives
+//     (td_operators_class.f:293-417): the strip kernel (k_strip,
+//     dim2d_strip.cu) over the border box in its masked modes -- primitives
 //     once per node, each face flux once with the interior Mattsson operators
 //     and the DIM flux formulas (every face of an interior_pt point lies
 //     between interior_pt / bc_interior_pt points, where the reference
@@ -118,7 +116,7 @@ int dim2d_time_dev_masked(const dim2d_params* p, int nx, int ny, const double* n
   a.rdy = 1.0 / dy;
   a.k = make_const(*p);
   a.c = strip_coef_of(a.k, a.rdx, a.rdy);
-  const cudaError_t e = launch_time_dev_masked(a, static_cast<cudaStream_t>(stream));
+  const cudaError_t e = launch_strip_masked(a, static_cast<cudaStream_t>(stream));
   if (e != cudaSuccess) return cuda_error(e, "time_dev_masked");
   return DIM2D_OK;
 }

@@ -80,6 +80,10 @@ __device__ __forceinline__ void cp_async16(double* smem, const double* gmem) {
   const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(sa), "l"(gmem) : "memory");
 }
+__device__ __forceinline__ void cp_async8(double* smem, const double* gmem) {
+  const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(sa), "l"(gmem) : "memory");
+}
 __device__ __forceinline__ void cp_async_commit() {
   asm volatile("cp.async.commit_group;\n" ::: "memory");
 }
@@ -120,6 +124,18 @@ struct RowCopy {
     cp_async16(to + dst, src);
     cp_async16(to + dst + 2 * RC, src + 2 * f.plane);
     if (lane < 4) cp_async16(to + edge_dst, src + edge);
+  }
+  // the same for MODE 3: any pitch and alignment, 8 bytes a copy.  The 8-byte
+  // form goes through L1, so its launches are plain ones: L1 is clean at their
+  // start, and nothing rewrites their input while they run.
+  __device__ __forceinline__ void narrow_state(const Field& f, const double* u, int c0, int row,
+                                               double* to, int lane) const {
+    const double* p = u + (size_t)row * f.pitch;
+    const int col = min(c0 - 2 + lane, f.nx - 1), edge_col = min(c0 + 30 + (lane & 1), f.nx - 1);
+#pragma unroll
+    for (int v = 0; v < 4; v++) cp_async8(to + v * RC + lane, p + v * f.plane + col);
+    if (lane < 8)
+      cp_async8(to + (lane >> 1) * RC + 32 + (lane & 1), p + (lane >> 1) * f.plane + edge_col);
   }
   // the row at distance d (in u^n) into the ring row at `to`
   __device__ __forceinline__ void un(const Field& f, ptrdiff_t d, double* to) const {
@@ -608,15 +624,19 @@ __device__ __forceinline__ void strip_warp(const StageArgs& a, int c0, int y0, i
 
   // rows y0-2 .. y0+2 into slots 0 .. 4, all in flight together
   RowCopy copy(a.uin, f, c0, y0 - 2, lane);
+  auto copy_state = [&](int row, double* to) {  // rows in order
+    if (MODE == 3) copy.narrow_state(f, a.uin, c0, row, to, lane);
+    else copy.state(f, to, lane);
+  };
 #pragma unroll
   for (int i = 0; i < 4; i++) {
-    copy.state(f, ring + i * ST_ROW, lane);
+    copy_state(y0 - 2 + i, ring + i * ST_ROW);
     copy.src += P;
   }
   cp_async_commit();
   // u^n of the row two below the state row being copied
   const ptrdiff_t un_row = (a.u0 - a.uin) - 2 * (ptrdiff_t)P;
-  copy.state(f, ring + 4 * ST_ROW, lane);
+  copy_state(y0 + 2, ring + 4 * ST_ROW);
   if (need_un) copy.un(f, un_row, uring);
   copy.src += P;
   cp_async_commit();
@@ -655,7 +675,7 @@ __device__ __forceinline__ void strip_warp(const StageArgs& a, int c0, int y0, i
   }
 
   const bool active = lane >= 1 && lane <= SW && x <= f.nx - 1 - BC &&
-                      (MODE != 2 || (x >= a.box_x0 && x <= a.box_x1));
+                      (MODE < 2 || (x >= a.box_x0 && x <= a.box_x1));
   // column of the cell's image in a ghost layer of a periodic or mirror side
   const bool images = MODE == 1 && (a.periodic || (UN != 2 && a.mirror));
   int ix2 = -1;
@@ -677,7 +697,7 @@ __device__ __forceinline__ void strip_warp(const StageArgs& a, int c0, int y0, i
   // the next row's copies: state row y0+3 into the slot of row y0-2
   __syncwarp();
   if (y0 + 1 < y1) {
-    copy.state(f, ring, lane);
+    copy_state(y0 + 3, ring);
     if (need_un) copy.un(f, un_row, uring + UN_ROW);
     copy.src += P;
   }
@@ -691,7 +711,7 @@ __device__ __forceinline__ void strip_warp(const StageArgs& a, int c0, int y0, i
 #pragma unroll 2
   for (int y = y0; y < y1; y++) {
     if (y + 2 < y1) {
-      copy.state(f, ring + ow, lane);
+      copy_state(y + 4, ring + ow);
       if (need_un) copy.un(f, un_row, uring + ouw);
       copy.src += P;
     }
@@ -753,7 +773,7 @@ __device__ __forceinline__ void strip_warp(const StageArgs& a, int c0, int y0, i
       for (int v = 0; v < 4; v++) ring[KEEP_AT + (y - y0) * ST_ROW + v * 32 + lane] = q[v];
     }
     // MODE 2 writes the interior_pt points of the layer map only
-    else if (active && (MODE != 2 || __ldg(a.mask + (size_t)y * P + x) == 1)) {
+    else if (active && (MODE < 2 || __ldg(a.mask + (size_t)y * P + x) == 1)) {
 #pragma unroll
       for (int v = 0; v < 4; v++) out[v * V] = q[v];
       // periodic_xy/bc_operators_class.f:156-199; mirrors change the sign of
@@ -939,9 +959,9 @@ __device__ __forceinline__ void strip_cta(const StageArgs& a, int b, int edge_ct
   }
   // MODE 2 (buffer-layer grid): strips over the border box, the first one
   // starting at an even column so that the rows' 16-byte pairs stay aligned
-  int c0 = (MODE == 2 ? (a.box_x0 & ~1) : BC) + (b % sx) * SW;
-  int y0 = (MODE == 2 ? a.box_y0 : BC) + (b / sx) * h;
-  const int ylast = MODE == 2 ? a.box_y1 : a.f.ny - BC - 1;
+  int c0 = (MODE >= 2 ? (a.box_x0 & ~1) : BC) + (b % sx) * SW;
+  int y0 = (MODE >= 2 ? a.box_y0 : BC) + (b / sx) * h;
+  const int ylast = MODE >= 2 ? a.box_y1 : a.f.ny - BC - 1;
   int y1 = min(y0 + h, ylast + 1);
   if (WALLS) {
     const WallRun run(a, b);
@@ -1343,7 +1363,10 @@ cudaError_t launch_strip_batch(BatchStageArgs& P, int kind, int shape, bool mixe
 
 // L(u) of a buffer-layer grid at its interior_pt points (MODE 2) over the
 // border box [box_x0, box_x1] x [box_y0, box_y1] (box_x0, box_y0 >= BC, so
-// every row and column read lies inside the grid).
+// every row and column read lies inside the grid).  MODE 3 where the layout
+// does not suit the rows' 16-byte copies (odd nx; 14.4 us on 2047 x 256 and
+// 6.2 us on 1001 x 100, where the tile kernel before it took 26.8 and 8.2; the
+// 16-byte form takes 12.0 us on 2048 x 256).
 cudaError_t launch_strip_masked(const StageArgs& a, cudaStream_t s) {
   int sx = (a.box_x1 - (a.box_x0 & ~1) + SW) / SW;
   const int rows = a.box_y1 - a.box_y0 + 1;
@@ -1351,8 +1374,11 @@ cudaError_t launch_strip_masked(const StageArgs& a, cudaStream_t s) {
   int edge_ctas = 0;
   StageArgs aa = a;
   void* args[] = {&aa, &edge_ctas, &sx, &h};
-  return launch_strips((const void*)k_strip<2, 0, E_NONE, false>,
-                       (unsigned)sx * (unsigned)((rows + h - 1) / h), s, args);
+  const unsigned blocks = (unsigned)sx * (unsigned)((rows + h - 1) / h);
+  if (strip_layout_ok(a))
+    return launch_strips((const void*)k_strip<2, 0, E_NONE, false>, blocks, s, args);
+  return cudaLaunchKernel((const void*)k_strip<3, 0, E_NONE, false>, dim3(blocks), dim3(32), args,
+                          WARP_DOUBLES * sizeof(double), s);
 }
 
 cudaError_t launch_strip_stage(const StageArgs& a, int mode, int shape, cudaStream_t s) {

@@ -101,3 +101,32 @@ def test_caller_layouts(F, preset, n, offset):
     got = dev.cpu().numpy().reshape(d["nodes"].shape)
     for v in range(4):
         assert np.abs(got[v] - ref[v]).max() <= 1e-12 * np.abs(ref[v]).max(), v
+
+
+@pytest.mark.parametrize("n,ny,offset", [(26, 9, 1), (27, 12, 0), (57, 20, 0), (61, 33, 0),
+                                         (62, 33, 1)])
+def test_masked_layouts(oracle, F, n, ny, offset):
+    """The masked time derivative where rows cannot be copied as 16-byte pairs:
+    odd nx, and even nx on an odd element, against the oracle (bar 1e-12)."""
+    import torch
+    d = workloads.domain(n, ny, T0=0.95, bubbles=[(0.0, 0.0, 0.2)], mach=0.05, bc="hedstrom_xy",
+                         li=0.2)
+    q, nx, nyy = d["nodes"], d["nx"], d["ny"]
+    dx, dy = d["x_map"][1] - d["x_map"][0], d["y_map"][1] - d["y_map"][0]
+    g = workloads.layer_map(nx, nyy, [(3, nx - 5, 3, nyy - 4)])
+    xb, yb = (3, nx - 3), (4, nyy - 2)
+    ref = np.full_like(q, 7.0)
+    oracle.compute_time_dev_masked(q, g, dx, dy, xb, yb, ref)
+    buf = torch.zeros(q.size + 2, dtype=torch.float64, device="cuda")
+    dev = buf[offset:offset + q.size]
+    dev.copy_(torch.from_numpy(q.reshape(-1)))
+    gd, td = torch.from_numpy(g).cuda(), torch.full(q.shape, 7.0, dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+    F.time_dev_masked(F.default_params(), nx, nyy, dev.data_ptr(), gd.data_ptr(), dx, dy, xb, yb,
+                      td.data_ptr())
+    torch.cuda.synchronize()
+    got, m = td.cpu().numpy(), g == 1
+    m[:yb[0] - 1] = m[yb[1]:] = m[:, :xb[0] - 1] = m[:, xb[1]:] = False
+    for v in range(4):
+        assert np.abs(got[v] - ref[v])[m].max() <= 1e-12 * np.abs(ref[v][m]).max(), v
+    assert np.all(got[:, ~m] == 7.0)
