@@ -119,6 +119,7 @@ cudaError_t group_stage(dim2d_batch* b, int g, const std::vector<int>& idx, int 
       d.mirror = h->mirror_sides;
       d.wall_runs = h->south_wall ? wall_run_count(h->f, h->open_mask) : 0;
       d.status = h->status;
+      if (h->south_wall) d.wc = wall_coef(h->wall, h->k, h->dx, h->dy);
     }
     cudaError_t e = launch_strip_batch(P, kind_of(g), shape, is_mixed(g), s);
     b->launches++;

@@ -35,6 +35,33 @@ __host__ __device__ __forceinline__ double wall_heat_flux(const WallConst& w, do
   return w.qmax * exp(-0.5 * (z * z));
 }
 
+// Constants of the wall columns' root function (dim2d_nodebc.cuh): computed
+// on the host once per stage launch (and per cell in a node pass), since the
+// solve's chain of instructions is what a stage of a small field waits for.
+struct WallCoef {
+  double rdx, rdy;  // inverse grid steps
+  double a1;        // 1/(We dy): dmddx_half / We
+  double a2;        // 1/(2 dy): interior gradient normal to the wall
+  double hwe;       // 1/(2 We)
+  double c38;       // 3/(8 cv_r)
+  double tq;        // temperature jump per heat flux, wall_xy_equilibrium_module.f:2295-2315
+  double C;         // 6 cos(angle) 2 sqrt(2)/(3 sqrt(We)) 9.6917.../3.97^3
+};
+__host__ __device__ __forceinline__ WallCoef wall_coef(const WallConst& w, const DimConst& k,
+                                                       double dx, double dy) {
+  WallCoef c;
+  c.rdx = 1.0 / dx;
+  c.rdy = 1.0 / dy;
+  c.a1 = 1.0 / (k.we * dy);
+  c.a2 = 0.5 / dy;
+  c.hwe = 0.5 / k.we;
+  c.c38 = 3.0 / (8.0 * k.cv_r);
+  c.tq = 0.5 * dy * k.re * k.pr * c.c38;
+  c.C = 6.0 * w.cos_angle * (2.0 * sqrt(2.0) / (3.0 * sqrt(k.we)) * 9.691686257306483) /
+        (3.97 * 3.97 * 3.97);
+  return c;
+}
+
 // Ghost sections integrated with the open (Hedstrom, bc_timedev) operator:
 // bits of StageArgs::open.  hedstrom_xy sets all of them; wall_S_open sets
 // N, W, E, NW, NE; half_wall_S_open sets N, E, NE (library_config.py:118-150).
@@ -128,6 +155,7 @@ struct StageArgs {
   int wall_runs;                       // south wall: runs of wall columns whose ghost cells
                                        // the launch solves (wall_run_count)
   unsigned int* status;                // wall root status word
+  WallCoef wc;                         // wall runs
   int reverse;                         // strips from the last to the first: every other
                                        // launch of a run, so that a stage starts on the
                                        // rows that the one before left in L2 (sustained,
@@ -291,6 +319,7 @@ struct BatchDomain {
   int open;                // OPEN_* mask of the time-integrated ghost sections
   int mirror, wall_runs;   // as StageArgs
   unsigned int* status;
+  WallCoef wc;
   int edge0, strip0, sx;   // first edge CTA, first strip CTA, strips per row
   StripCoef<double> c;
 };
@@ -304,6 +333,7 @@ struct BatchStageArgs {
   int edge_ctas;   // edge runs of all domains, placed before all strips
   BatchDomain d[BATCH_MAX];
 };
+static_assert(sizeof(BatchStageArgs) <= 32764, "kernel parameters");
 
 // boundary kinds of a batched stage launch; BK_WALL launches also integrate
 // the open sections of wall_S_open / half_wall_S_open members (their

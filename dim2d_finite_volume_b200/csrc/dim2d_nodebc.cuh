@@ -67,9 +67,8 @@ struct WallRoot {
   double md2;  // md_x(1): second interior density
   double my0, my1;
   double vx, vy, Ed;
-  double dxn, dyt;  // delta_x (normal), delta_y (tangential)
+  double ir1;  // 1/md_x(2)
   double q;
-  double cosang;
   int gt;  // WallGrad of the tangential density gradient (get_dmd_dx, :2433-2461)
 };
 
@@ -90,33 +89,30 @@ __host__ __device__ __forceinline__ double md_liq(double T) { return 1.0 + 2.06 
 // value differs from the reference's evaluation order by rounding only.
 struct WallRootFn {
   double md1, md2;
-  double a1;    // 1/(We delta_x): dmddx_half / We
-  double a2;    // 1/(2 delta_x): interior gradient normal to the wall
+  double a1, a2, C, c38;  // WallCoef
   double gy2;   // square of the tangential density gradient (get_dmd_dx type of the column)
   double base;  // Ed/md - |v|^2/2 + 3 md, the temperature without its gradient term
   double cw;    // 1/(2 We md)
-  double c38;   // 3/(8 cv_r)
-  double tq;    // temperature jump of the heat flux, :2295-2315
-  double C;
+  double tq;    // temperature jump of the heat flux
 };
 
-__host__ __device__ __forceinline__ WallRootFn wall_root_fn(const WallRoot& c, const DimConst& k) {
+__host__ __device__ __forceinline__ WallRootFn wall_root_fn(const WallRoot& c,
+                                                            const WallCoef& wc) {
   WallRootFn w;
   double gy;
-  if (c.gt == WG_L0) gy = (c.my1 - c.md1) / c.dyt;
-  else if (c.gt == WG_R0) gy = (c.md1 - c.my0) / c.dyt;
-  else gy = (c.my1 - c.my0) / (2.0 * c.dyt);
+  if (c.gt == WG_L0) gy = (c.my1 - c.md1) * wc.rdx;
+  else if (c.gt == WG_R0) gy = (c.md1 - c.my0) * wc.rdx;
+  else gy = (c.my1 - c.my0) * (0.5 * wc.rdx);
   w.md1 = c.md1;
   w.md2 = c.md2;
-  w.a1 = 1.0 / (k.we * c.dxn);
-  w.a2 = 0.5 / c.dxn;
+  w.a1 = wc.a1;
+  w.a2 = wc.a2;
+  w.C = wc.C;
+  w.c38 = wc.c38;
   w.gy2 = gy * gy;
-  w.base = c.Ed / c.md1 - 0.5 * (c.vx * c.vx + c.vy * c.vy) + 3.0 * c.md1;
-  w.cw = 0.5 / (k.we * c.md1);
-  w.c38 = 3.0 / (8.0 * k.cv_r);
-  w.tq = 0.5 * c.dxn * k.re * k.pr * w.c38 * c.q;
-  w.C = 6.0 * c.cosang * (2.0 * sqrt(2.0) / (3.0 * sqrt(k.we)) * 9.691686257306483) /
-        (3.97 * 3.97 * 3.97);
+  w.base = c.Ed * c.ir1 - 0.5 * (c.vx * c.vx + c.vy * c.vy) + 3.0 * c.md1;
+  w.cw = wc.hwe * c.ir1;
+  w.tq = wc.tq * c.q;
   return w;
 }
 
@@ -137,28 +133,22 @@ __host__ __device__ __forceinline__ bool validated(double a, double b) { return 
 // *status gets 1 (no bracket), 2 (not bracketed), 3 (no convergence) or
 // 4 (bracketing error).
 //
-// The sequence of trial points and tests is the reference's; only the order
-// of evaluation is changed for latency (one thread per wall column, so the
-// chain of dependent root-function calls is the kernel's duration): the
-// bracket ends, the guess and the first scan pair are evaluated together,
-// before the tests that use them, and Ridders' method starts from the
-// function values of its bracket ends already computed (the reference
-// evaluates them again; the function is deterministic, so the values and
-// the result are the same).
+// The sequence of trial points and tests is the reference's; Ridders' method
+// starts from the function values of its bracket ends already computed (the
+// reference evaluates them again; the function is deterministic, so the
+// values and the result are the same).
 __host__ __device__ inline double wall_root(const WallRoot& c, double T_guess, double md_guess,
-                                     const DimConst& k, unsigned int* status) {
-  const WallRootFn w = wall_root_fn(c, k);
+                                     const WallCoef& wc, unsigned int* status) {
+  const WallRootFn w = wall_root_fn(c, wc);
   double xl = md_vap(T_guess), xh = md_liq(T_guess);
-  const double dmd_l = md_guess / 100.0, dmd_r = (3.0 - md_guess) / 100.0;
-  const double a1 = md_guess - 1 * dmd_l, b1 = md_guess + 1 * dmd_r;
   double fl = wall_root_f(w, xl), fh = wall_root_f(w, xh);
-  const double fmd = wall_root_f(w, md_guess);
-  const double fa1 = wall_root_f(w, a1), fb1 = wall_root_f(w, b1);
   if (same_sign(fl, fh)) {
+    const double dmd_l = md_guess / 100.0, dmd_r = (3.0 - md_guess) / 100.0;
+    const double fmd = wall_root_f(w, md_guess);
     bool found = false;
     for (int j = 1; j <= 99 && !found; j++) {
       const double a = md_guess - j * dmd_l, b = md_guess + j * dmd_r;
-      const double fa = j == 1 ? fa1 : wall_root_f(w, a);
+      const double fa = wall_root_f(w, a);
       if (!same_sign(fa, fmd)) {
         xl = a;
         xh = md_guess;
@@ -167,7 +157,7 @@ __host__ __device__ inline double wall_root(const WallRoot& c, double T_guess, d
         found = true;
         break;
       }
-      const double fb = j == 1 ? fb1 : wall_root_f(w, b);
+      const double fb = wall_root_f(w, b);
       if (!same_sign(fb, fmd)) {
         xl = md_guess;
         xh = b;
@@ -242,39 +232,36 @@ struct WallIn {
 struct WallOut {
   double r, r0, mx, my;  // ghost row 1: density, momenta; ghost row 0: density
 };
-// x = the column's coordinate; gt = WallGrad type of its tangential gradients
-__host__ __device__ __forceinline__ WallOut wall_column(const WallIn& in, int gt, double x,
-                                                        double dx, double dy,
-                                                        const WallConst& wall, const DimConst& k,
+// gt = WallGrad type of its tangential gradients, q = its heat flux
+__host__ __device__ __forceinline__ WallOut wall_column(const WallIn& in, int gt, double q,
+                                                        const WallCoef& wc,
                                                         unsigned int* status) {
   // temperature guess, temperature_eff dim2d_prim_module.f:652-691
   double gx;
-  if (gt == WG_L0) gx = 1.0 / dx * (-in.gr + in.gre);
-  else if (gt == WG_R0) gx = 1.0 / dx * (-in.grw + in.gr);
-  else gx = 0.5 / dx * (-in.grw + in.gre);
-  const double gy = 0.5 / dy * (-in.grs + in.grn);
-  const double vx = in.gmx / in.gr, vy = in.gmy / in.gr;
-  const double teff = 1.0 / in.gr * (in.gE - 0.5 * in.gr * (vx * vx + vy * vy) -
-                                     0.5 / k.we * (gx * gx + gy * gy) + 3.0 * (in.gr * in.gr));
-  const double Tg = 3.0 / (8.0 * k.cv_r) * teff;
+  if (gt == WG_L0) gx = wc.rdx * (-in.gr + in.gre);
+  else if (gt == WG_R0) gx = wc.rdx * (-in.grw + in.gr);
+  else gx = 0.5 * wc.rdx * (-in.grw + in.gre);
+  const double gy = 0.5 * wc.rdy * (-in.grs + in.grn);
+  const double ig = 1.0 / in.gr;
+  const double vx = in.gmx * ig, vy = in.gmy * ig;
+  const double teff = ig * (in.gE - 0.5 * in.gr * (vx * vx + vy * vy) -
+                            wc.hwe * (gx * gx + gy * gy) + 3.0 * (in.gr * in.gr));
   WallRoot c;
   c.md1 = in.r1;
   c.md2 = in.r2;
   c.my0 = in.rw;
   c.my1 = in.re;
   c.gt = gt;
-  c.vx = -in.my1 / in.r1;
-  c.vy = in.mx1 / in.r1;
+  c.ir1 = 1.0 / in.r1;
+  c.vx = -in.my1 * c.ir1;
+  c.vy = in.mx1 * c.ir1;
   c.Ed = in.E1;
-  c.dxn = dy;
-  c.dyt = dx;
-  c.q = wall_heat_flux(wall, x);
-  c.cosang = wall.cos_angle;
+  c.q = q;
   WallOut o;
-  o.r = wall_root(c, Tg, in.grs, k, status);
+  o.r = wall_root(c, wc.c38 * teff, in.grs, wc, status);
   o.r0 = in.r2 + 3.0 * (-in.r1 + o.r);   // :1439-1465 (high-order extrapolation)
-  o.mx = -1.0 * in.mx1 / in.r1 * o.r;    // sign_trans
-  o.my = 1.0 * in.my1 / in.r1 * o.r;     // sign_normal
+  o.mx = -c.vy * o.r;                    // sign_trans
+  o.my = -c.vx * o.r;                    // sign_normal
   return o;
 }
 
@@ -388,7 +375,8 @@ __host__ __device__ inline void node_bc_cell(const NodeBcArgs& a, int m) {
       in.re = x + 1 >= nx - BC && !a.open_e ? ld(u, f, 0, mirror_lo_hi(x + 1, nx), 2)
                                             : ld(u, f, 0, x + 1, 2);
     unsigned int st = 0;
-    const WallOut o = wall_column(in, gt, a.xmap0 + x * a.dx, a.dx, a.dy, a.wall, k, &st);
+    const WallOut o = wall_column(in, gt, wall_heat_flux(a.wall, a.xmap0 + x * a.dx),
+                                  wall_coef(a.wall, k, a.dx, a.dy), &st);
     if (st && a.status) {
 #ifdef __CUDA_ARCH__
       atomicOr(a.status, st);

@@ -39,6 +39,7 @@ StageArgs make_stage_args(const dim2d_handle* h, const double* uin, double* uout
   a.mirror = h->mirror_sides;
   a.wall_runs = h->south_wall ? wall_run_count(h->f, h->open_mask) : 0;
   a.status = h->status;
+  if (h->south_wall) a.wc = wall_coef(h->wall, h->k, h->dx, h->dy);
   a.apart = open_runs_apart(a);
   a.wall = h->wall;
   a.k = h->k;

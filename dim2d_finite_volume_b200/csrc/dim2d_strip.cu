@@ -919,7 +919,8 @@ __device__ __forceinline__ void wall_columns(const StageArgs& a, const WallRun& 
   if (!mine) return;
   const int gt = x == 0 ? WG_L0 : (x == f.nx - 1 ? WG_R0 : WG_CENTRED);
   unsigned int st = 0;
-  const WallOut o = wall_column(in, gt, a.xmap0 + x * a.dx, a.dx, a.dy, a.wall, a.k, &st);
+  const WallOut o =
+      wall_column(in, gt, wall_heat_flux(a.wall, a.xmap0 + x * a.dx), a.wc, &st);
   if (st) atomicOr(a.status, st);
   double* u = a.uout + x;
   u[P] = o.r;
@@ -1017,6 +1018,7 @@ __device__ __forceinline__ StageArgs batch_stage_args(const BatchStageArgs& P, i
   a.mirror = d.mirror;
   a.wall_runs = d.wall_runs;
   a.status = d.status;
+  a.wc = d.wc;
   a.apart = a.reverse = 0;
   a.mixed = 0;
   a.t = 0.0;
