@@ -116,6 +116,7 @@ cudaError_t group_stage(dim2d_batch* b, int g, const std::vector<int>& idx, int 
       d.wall_s = h->south_wall;
       d.open = h->open_mask;
       d.c = strip_coef_of(h->k, h->rdx, h->rdy);
+      d.cf = strip_coef_f32(d.c);
       d.mirror = h->mirror_sides;
       d.wall_runs = h->south_wall ? wall_run_count(h->f, h->open_mask) : 0;
       d.status = h->status;

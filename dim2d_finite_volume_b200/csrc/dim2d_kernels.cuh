@@ -322,6 +322,7 @@ struct BatchDomain {
   WallCoef wc;
   int edge0, strip0, sx;   // first edge CTA, first strip CTA, strips per row
   StripCoef<double> c;
+  StripCoef<float> cf;
 };
 
 struct BatchStageArgs {
@@ -374,6 +375,7 @@ struct PDomain {
   int nn;                                            // node items per stage (0: no pass)
   unsigned int* status;                              // wall root status word
   StripCoef<double> c;
+  StripCoef<float> cf;
 };
 
 struct PItem {

@@ -165,6 +165,7 @@ int persist_build(PersistPlan& pl, const std::vector<dim2d_handle*>& hs,
     d.open_n = h->open_n;
     d.status = h->status;
     d.c = strip_coef_of(h->k, h->rdx, h->rdy);
+    d.cf = strip_coef_f32(d.c);
     d.sx = (h->f.nx - 2 * BC + STRIP_COLS - 1) / STRIP_COLS;
     d.nb = band_count(h->f.ny - 2 * BC, rows);
     d.band0 = (int)sg.size();

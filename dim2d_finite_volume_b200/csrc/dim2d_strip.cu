@@ -708,7 +708,7 @@ __device__ __forceinline__ void strip_warp(const StageArgs& a, int c0, int y0, i
   int o1 = 3 * ST_ROW, o2 = 4 * ST_ROW, ow = ST_ROW, ou = 0, ouw = 2 * UN_ROW;
 
   // r0/mx0/my0/e0 = state row y, r1 = density of row y+1
-#pragma unroll 2
+#pragma unroll(UN == 2 ? 1 : 2)  // (persistent kernel: registers)
   for (int y = y0; y < y1; y++) {
     if (y + 2 < y1) {
       copy_state(y + 4, ring + ow);
@@ -1027,7 +1027,7 @@ __device__ __forceinline__ StageArgs batch_stage_args(const BatchStageArgs& P, i
   a.wall = P.wall;
   a.k = P.k;
   a.c = d.c;
-  if (MIX) a.cf = strip_coef_f32(d.c);
+  if (MIX) a.cf = d.cf;
   return a;
 }
 
@@ -1108,42 +1108,46 @@ __device__ bool wait_done(const PersistArgs& P, const unsigned long long* done,
   return false;
 }
 
+// Stage arguments of an item, built by the warp in shared memory: strips and
+// ghost runs read them from there as they need them.  In registers, and with
+// 16 warps per SM, they spilled 500 bytes in the strips' loop (64-domain FP64
+// batch 1235 us per step); from shared memory 912 at 16 warps (144 bytes), 651
+// at 12 (158 registers, none).
 template <bool MIX>
-__device__ __forceinline__ StageArgs persist_stage_args(const PersistArgs& P, const PDomain& d,
-                                                        int step, int st) {
+__device__ __forceinline__ void persist_stage_args(const PersistArgs& P, const PDomain& d,
+                                                   int step, int st, StageArgs& a) {
+  __syncwarp();  // the warp is done with its item before
+  const int lane = threadIdx.x & 31;
+  constexpr int NC = sizeof(StripCoef<double>) / sizeof(double);
+  if (lane < NC) {
+    reinterpret_cast<double*>(&a.c)[lane] = reinterpret_cast<const double*>(&d.c)[lane];
+    if (MIX) reinterpret_cast<float*>(&a.cf)[lane] = reinterpret_cast<const float*>(&d.cf)[lane];
+  }
   const int odd = (P.step0 + step) & 1;
   double* X = odd ? d.buf[1] : d.buf[0];  // u^n
   double* Y = odd ? d.buf[0] : d.buf[1];
-  StageArgs a;
-  a.uin = st == 1 ? X : (st == 2 ? Y : d.buf[2]);
-  a.u0 = X;
-  a.uout = st == 2 ? d.buf[2] : Y;
-  a.f = d.f;
-  a.dx = d.dx;
-  a.dy = d.dy;
-  a.rdx = d.rdx;
-  a.rdy = d.rdy;
-  a.dt = d.dt * P.dt_scale;
-  a.b = st == 2 ? 0.75 : (st == 3 ? 1.0 / 3.0 : 0.0);  // rk3tvd_steps_module.f:225,444
-  a.stage = st;
-  a.periodic = d.periodic;
-  a.wall_s = d.wall_s;
-  a.variant = 0;
-  a.open = d.open;
-  a.mixed = 0;
-  a.t = 0.0;
-  a.xmap0 = d.xmap0;
-  a.ymap0 = d.ymap0;
-  a.mirror = a.wall_runs = 0;  // its items
-  a.status = nullptr;
-  a.apart = a.reverse = 0;
-  a.mask = nullptr;
-  a.box_x0 = a.box_x1 = a.box_y0 = a.box_y1 = 0;
-  a.wall = P.wall;
-  a.k = P.k;
-  a.c = d.c;
-  if (MIX) a.cf = strip_coef_f32(d.c);
-  return a;
+  if (lane == 0) {
+    a.uin = st == 1 ? X : (st == 2 ? Y : d.buf[2]);
+    a.u0 = X;
+    a.uout = st == 2 ? d.buf[2] : Y;
+    a.f = d.f;
+    a.dx = d.dx;
+    a.dy = d.dy;
+    a.rdx = d.rdx;
+    a.rdy = d.rdy;
+    a.dt = d.dt * P.dt_scale;
+    a.b = st == 2 ? 0.75 : (st == 3 ? 1.0 / 3.0 : 0.0);  // rk3tvd_steps_module.f:225,444
+    a.stage = st;
+    a.periodic = d.periodic;
+    a.wall_s = d.wall_s;
+    a.open = d.open;
+    a.xmap0 = d.xmap0;
+    a.mirror = a.wall_runs = 0;  // its node items
+    a.apart = a.reverse = 0;
+    a.wall = P.wall;
+    a.k = P.k;
+  }
+  __syncwarp();
 }
 
 __device__ __forceinline__ NodeBcArgs persist_node_args(const PersistArgs& P, const PDomain& d,
@@ -1180,9 +1184,11 @@ __device__ __forceinline__ bool wait_band(const PersistArgs& P, const PDomain& d
 }
 
 template <bool MIX>
-__global__ void __launch_bounds__(32 * PW, 8) k_batch_persistent(const __grid_constant__ PersistArgs P) {
+__global__ void __launch_bounds__(32 * PW, 6) k_batch_persistent(const __grid_constant__ PersistArgs P) {
   const int lane = threadIdx.x & 31;
   const unsigned long long total = (unsigned long long)P.items_per_step * P.nsteps;
+  __shared__ StageArgs args[PW];
+  StageArgs& a = args[threadIdx.x >> 5];
   for (;;) {
     unsigned long long it = 0;
     if (lane == 0) it = atomicAdd(P.next, 1ull);
@@ -1231,7 +1237,7 @@ __global__ void __launch_bounds__(32 * PW, 8) k_batch_persistent(const __grid_co
     // a wait that ran out stops the warp (the launch is aborted)
     if (!__all_sync(0xffffffffu, ok)) break;
     if (item.type == PI_STRIP) {
-      const StageArgs a = persist_stage_args<MIX>(P, d, step, item.stage);
+      persist_stage_args<MIX>(P, d, step, item.stage, a);
       const int c0 = BC + (item.index % d.sx) * SW;
       const int y0 = BC + item.band * P.h_rows;
       // the last band runs to the last interior row (it absorbs a remainder
@@ -1240,7 +1246,7 @@ __global__ void __launch_bounds__(32 * PW, 8) k_batch_persistent(const __grid_co
       const int y1 = item.band == d.nb - 1 ? d.f.ny - BC : y0 + P.h_rows;
       strip_warp<1, 2, MIX>(a, c0, y0, y1);
     } else if (item.type == PI_GHOST) {
-      const StageArgs a = persist_stage_args<false>(P, d, step, item.stage);
+      persist_stage_args<false>(P, d, step, item.stage, a);
       const int side = item.index >> 24;
       if (side < 4)
         open_edge_run<1>(a, side, item.index >> 20 & 1, item.index & 0xfffff, item.count);
