@@ -272,12 +272,12 @@ int rk3_steps(dim2d_handle* h, double dt, int nsteps) {
     h->graph_dt = dt;
   }
   for (int s = 0; s < nsteps;) {
-    // stage 1 writes B (and, a step on, A): pending asynchronous copies of
-    // them must land first
-    const int size = graph_size_for(nsteps - s);
+    // stage 1 writes B: a pending asynchronous copy of B must land first.  One
+    // of A overlaps the first step; the second writes A.
+    const bool copying = h->copy_pending && h->copy_src == h->A;
+    const int size = graph_size_for(copying ? 1 : nsteps - s);
     const int n = graphs ? GRAPH_STEPS[size] : 1;
     cudaError_t ew = wait_copy_if(h, h->B);
-    if (ew == cudaSuccess && n > 1) ew = wait_copy_if(h, h->A);
     if (ew != cudaSuccess) return cuda_error(ew, "step");
     if (graphs) {
       StepGraph* const slots = h->graph[size];
