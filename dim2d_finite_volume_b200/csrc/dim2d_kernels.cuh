@@ -162,7 +162,6 @@ struct StageArgs {
                                        // us per step: 2048^2 open 269 -> 260, mixed wall
                                        // 256 -> 249; evicting dead inputs first: no gain;
                                        // batches, whose kinds overlap: 1 % slower, never)
-  int apart;                           // its ghost cells take the launch before (open_runs_apart)
   const int* __restrict__ mask;        // time derivative of a buffer-layer grid: its
                                        // grdpts_id map, written only where it is
                                        // interior_pt (1) inside [box_x0, box_x1] x
@@ -237,7 +236,7 @@ cudaError_t launch_interior_stage(const StageArgs& a, cudaStream_t s);
 // strip kernel (dim2d_strip.cu); mode 0 = L(u), 1 = stage update; shape 0..4 =
 // strips of 8, 16, 32, 4, 2 rows, SHAPE_BY_SIZE = by the field's size
 cudaError_t launch_strip_stage(const StageArgs& a, int mode, int shape, cudaStream_t s);
-// the ghost runs of open_runs_apart(a); launch_strip_stage follows on `s`
+// the ghost runs of the sections in a.open alone, as a launch of their own
 cudaError_t launch_open_runs(const StageArgs& a, int mode, cudaStream_t s);
 // The strip kernels read state and u^n rows as 16-byte pairs: they need an
 // even pitch and 16-byte aligned planes.  Fields allocated by the library
@@ -252,16 +251,10 @@ constexpr int SHAPE_BY_SIZE = -1;
 inline int strip_shape_of(const StageArgs& a) {
   return a.variant >= 1 && a.variant <= 5 ? a.variant - 1 : SHAPE_BY_SIZE;
 }
-// 1 if the ghost cells of an open field take a launch of their own: tile
-// kernel, and variant 0 on hedstrom_xy, whose two kernels per stage callers
-// count (dim2d_launch_count); there the strips are a programmatic dependent
-// of the ghost launch and overlap it (launch_strip_stage)
-inline bool open_runs_apart(const StageArgs& a) {
-  return a.open == OPEN_ALL && a.variant == 0 && strip_layout_ok(a);
-}
-inline bool stage_fuses_open(const StageArgs& a) {
-  return a.open && strip_layout_ok(a) && !open_runs_apart(a);
-}
+// 1 if the stage launch of `a` integrates its open sections too
+inline bool stage_fuses_open(const StageArgs& a) { return a.open && strip_layout_ok(a); }
+// sections a.open without the edges S, N, W, E: the corner cells
+constexpr int OPEN_CORNERS = OPEN_SW | OPEN_SE | OPEN_NW | OPEN_NE;
 // variants: 0 = strips of a height chosen by the field's size, 1..5 = strip
 // shapes 0..4, 6 = the persistent kernel (a whole step per launch,
 // dim2d_persist.cu; its time derivative alone runs as variant 0)

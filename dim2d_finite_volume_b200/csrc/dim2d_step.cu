@@ -40,7 +40,6 @@ StageArgs make_stage_args(const dim2d_handle* h, const double* uin, double* uout
   a.wall_runs = h->south_wall ? wall_run_count(h->f, h->open_mask) : 0;
   a.status = h->status;
   if (h->south_wall) a.wc = wall_coef(h->wall, h->k, h->dx, h->dy);
-  a.apart = open_runs_apart(a);
   a.wall = h->wall;
   a.k = h->k;
   a.c = strip_coef_of(h->k, h->rdx, h->rdy);
@@ -127,18 +126,23 @@ int check_status(dim2d_handle* h) {
 }
 
 cudaError_t launch_stage_work(dim2d_handle* h, const StageArgs& a, int mode) {
-  cudaError_t e = cudaSuccess;
-  const bool apart = a.apart != 0;
-  if (apart) {
-    e = launch_open_runs(a, mode, h->stream);
-    h->launches++;
-    if (e != cudaSuccess) return e;
-  }
+  // Callers count two kernels per stage on an untuned hedstrom_xy field
+  // (dim2d_launch_count): there the corner cells follow in a launch of their own.
+  const bool corners_apart = a.open == OPEN_ALL && a.variant == 0 && !h->uncounted;
+  StageArgs first = a;
+  if (corners_apart) first.open &= ~OPEN_CORNERS;
   prof_begin(h);
-  e = mode == 0 ? launch_time_dev(a, h->stream) : launch_interior_stage(a, h->stream);
+  cudaError_t e =
+      mode == 0 ? launch_time_dev(first, h->stream) : launch_interior_stage(first, h->stream);
   prof_end(h);
   h->launches++;
-  if (e == cudaSuccess && a.open && !apart && !stage_fuses_open(a)) {
+  if (e != cudaSuccess || !a.open) return e;
+  if (corners_apart) {
+    StageArgs corners = a;
+    corners.open = OPEN_CORNERS;
+    e = launch_open_runs(corners, mode, h->stream);
+    h->launches++;
+  } else if (!stage_fuses_open(a)) {
     e = launch_open_ghosts(a, mode, h->stream);
     h->launches++;
   }

@@ -56,10 +56,9 @@ constexpr int WARPS = 16;       // resident warps per SM (one warp per CTA, <= 1
 // its stream: it lets its own dependent start before it ends and waits for the
 // launch before it, complete and visible, before its first read
 // (griddepcontrol.wait), so that launch latency and block scheduling overlap
-// that launch's end.  Strips after their own ghost runs (StageArgs::apart)
-// start without waiting: the runs have themselves waited for the launch whose
-// output both read before they let the strips start, and write other cells;
-// the first CTA waits at its end, so that the strips' end implies the runs'.
+// that launch's end.  The wait is what makes that launch's output visible: no
+// kernel reads or writes a state before it, whatever ran in between (a launch
+// that let its dependents start gives them no ordering by that alone).
 
 template <typename T>
 __device__ __forceinline__ T from_left(T v) {
@@ -612,7 +611,7 @@ __device__ __forceinline__ void strip_warp(const StageArgs& a, int c0, int y0, i
   const StripCoef<T>& c = coef_of(a, T(0));
   const bool need_un = MODE == 1 && (UN == 2 ? a.stage != 1 : UN == 1);
 
-  if (UN != 2 && !a.apart) wait_for_launch_before();
+  if (UN != 2) wait_for_launch_before();
 
   // the lane's column (columns past the field are not stored); its place in
   // a ring row
@@ -984,10 +983,9 @@ __global__ void __launch_bounds__(32, WARPS) k_strip(const __grid_constant__ Sta
   int b = blockIdx.x;
   if (a.reverse && b >= edge_ctas) b = edge_ctas + (int)gridDim.x - 1 - b;
   strip_cta<MODE, UN, EDGES, MIX>(a, b, edge_ctas, sx, h);
-  if (EDGES == E_NONE && a.apart && blockIdx.x == 0) wait_for_launch_before();
 }
 
-// the ghost runs alone (open_runs_apart)
+// ghost runs alone (launch_stage_work: the corner cells of an untuned open field)
 template <int MODE>
 __global__ void __launch_bounds__(32) k_open_runs(const __grid_constant__ StageArgs a) {
   wait_for_launch_before();
@@ -1019,7 +1017,7 @@ __device__ __forceinline__ StageArgs batch_stage_args(const BatchStageArgs& P, i
   a.wall_runs = d.wall_runs;
   a.status = d.status;
   a.wc = d.wc;
-  a.apart = a.reverse = 0;
+  a.reverse = 0;
   a.mixed = 0;
   a.t = 0.0;
   a.xmap0 = d.xmap0;
@@ -1143,7 +1141,7 @@ __device__ __forceinline__ void persist_stage_args(const PersistArgs& P, const P
     a.open = d.open;
     a.xmap0 = d.xmap0;
     a.mirror = a.wall_runs = 0;  // its node items
-    a.apart = a.reverse = 0;
+    a.reverse = 0;
     a.wall = P.wall;
     a.k = P.k;
   }
@@ -1394,7 +1392,7 @@ cudaError_t launch_strip_stage(const StageArgs& a, int mode, int shape, cudaStre
   int sx = strips_across(a.f);
   int h = rows_of(shape, [&](int rows) { return (long long)sx * strips_up(a.f, rows); });
   const int walls = mode == 1 ? a.wall_runs : 0;
-  int edge_ctas = walls + (a.apart ? 0 : open_run_count(a.f, a.open));
+  int edge_ctas = walls + open_run_count(a.f, a.open);
   const int edges = walls ? E_WALL : (edge_ctas ? E_OPEN : E_NONE);
   const void* fn = a.mixed ? strip_fn<true>(mode, a.stage != 1, edges)
                            : strip_fn<false>(mode, a.stage != 1, edges);
