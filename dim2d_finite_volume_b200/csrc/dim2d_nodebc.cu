@@ -1,6 +1,5 @@
-// dim2d_nodebc.cu -- launches of the node boundary pass (one field, or
-// every domain of a batch); the per-cell work is node_bc_cell() in
-// dim2d_nodebc.cuh.
+// dim2d_nodebc.cu -- launch of the node boundary pass of one field; the
+// per-cell work is node_bc_cell() in dim2d_nodebc.cuh.
 #include "dim2d_nodebc.cuh"
 
 namespace dim2d {

@@ -40,9 +40,6 @@
 // cells (open_run, one warp per run): they take the first CTAs of the grid, so
 // that they overlap the strips.  Ghost and interior cells read the same input
 // and write disjoint cells.
-// the ghost-cell and node-pass code of this file runs inside the persistent
-// kernel, whose inputs change during the launch: coherent loads
-#define DIM2D_COHERENT_LOADS
 #include "dim2d_nodebc.cuh"
 
 namespace dim2d {
@@ -772,7 +769,7 @@ __device__ __forceinline__ void strip_warp(const StageArgs& a, int c0, int y0, i
       for (int v = 0; v < 4; v++) ring[KEEP_AT + (y - y0) * ST_ROW + v * 32 + lane] = q[v];
     }
     // MODE 2 writes the interior_pt points of the layer map only
-    else if (active && (MODE < 2 || __ldg(a.mask + (size_t)y * P + x) == 1)) {
+    else if (active && (MODE < 2 || __ldcg(a.mask + (size_t)y * P + x) == 1)) {
 #pragma unroll
       for (int v = 0; v < 4; v++) out[v * V] = q[v];
       // periodic_xy/bc_operators_class.f:156-199; mirrors change the sign of

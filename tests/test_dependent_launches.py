@@ -28,3 +28,15 @@ def test_no_wait_depends_on_the_launch():
             names = set(re.findall(r"[A-Za-z_][\w.]*", m["cond"] or ""))
             assert names <= TEMPLATE, (name, m[0])
     assert found >= 5
+
+
+def test_no_dependent_reads_through_the_read_only_path():
+    """ld.global.nc is specified for data that nothing writes from a kernel's
+    start to its end; a dependent starts before its input is complete.  The
+    sources that may use it hold plain launches only."""
+    plain = {"dim2d_open.cuh", "dim2d_interior.cu"}
+    for name, text in _sources():
+        if name in plain:
+            assert "wait_for_launch_before();" not in text, name
+        else:
+            assert "__ldg(" not in text and "ld.global.nc" not in text, name
