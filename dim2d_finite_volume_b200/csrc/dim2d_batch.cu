@@ -138,20 +138,35 @@ std::vector<int> members_of(const dim2d_batch* b, int g) {
 
 // `steps` steps of every group, each group's chain on its own stream forked
 // from b->stream (so the chains overlap, and one group need not wait for
-// another between its steps); joined back into b->stream.
+// another between its steps); joined back into b->stream.  Issued stage by
+// stage, so that no group's chain waits for the launches of another's.
 cudaError_t launch_steps(dim2d_batch* b, int steps) {
   cudaError_t e = cudaEventRecord(b->fork, b->stream);
+  std::vector<int> idx[NGROUPS];
   for (int g = 0; g < NGROUPS && e == cudaSuccess; g++) {
-    const std::vector<int> idx = members_of(b, g);
-    if (idx.empty()) continue;
-    e = cudaStreamWaitEvent(b->side[g], b->fork, 0);
-    for (int k = 0; k < 3 * steps && e == cudaSuccess; k++)
-      e = group_stage(b, g, idx, k % 3 + 1, b->shape[g], 1.0, b->side[g], k / 3 & 1);
-    if (e == cudaSuccess) e = cudaEventRecord(b->join[g], b->side[g]);
+    idx[g] = members_of(b, g);
+    if (!idx[g].empty()) e = cudaStreamWaitEvent(b->side[g], b->fork, 0);
+  }
+  for (int k = 0; k < 3 * steps; k++)
+    for (int g = 0; g < NGROUPS && e == cudaSuccess; g++)
+      if (!idx[g].empty())
+        e = group_stage(b, g, idx[g], k % 3 + 1, b->shape[g], 1.0, b->side[g], k / 3 & 1);
+  for (int g = 0; g < NGROUPS && e == cudaSuccess; g++) {
+    if (idx[g].empty()) continue;
+    e = cudaEventRecord(b->join[g], b->side[g]);
     if (e == cudaSuccess) e = cudaStreamWaitEvent(b->stream, b->join[g], 0);
   }
   return e;
 }
+
+// Runs that are launched directly before the graph they could have replayed is
+// captured.  A capture costs what three to five direct runs lose against
+// replays (8 steps of three 64^2 fields of different kinds: 490 us launched
+// directly, 242 replayed, 1090 with the capture; 64 fields of 128^2: 1270,
+// 1110, 1910), and a change of members, dt or shapes drops the graphs: captured
+// at first use, runs of 8 to 15 steps of a new batch of few small fields took
+// longer than with graphs of one step.
+constexpr int GRAPH_AFTER = 4;
 
 void swap_members(dim2d_batch* b) {
   for (dim2d_handle* h : b->m) std::swap(h->A, h->B);
@@ -404,21 +419,17 @@ int dim2d_batch_step(dim2d_batch* b, int nsteps) {
   }
   for (int s = 0; s < nsteps;) {
     const int size = graph_size_for(nsteps - s);
-    int n = GRAPH_STEPS[size];
-    StepGraph* g = nullptr;
-    if (b->use_graphs) {
-      g = &b->graph[size][b->parity];
-      if (!g->exec) {
-        int rc = capture(b, *g, n);
-        if (rc && rc != DIM2D_ERR_UNSUPPORTED) return rc;
-      }
+    const int n = GRAPH_STEPS[size];
+    StepGraph& g = b->graph[size][b->parity];
+    if (b->use_graphs && !g.exec && g.asked++ >= GRAPH_AFTER) {
+      int rc = capture(b, g, n);
+      if (rc && rc != DIM2D_ERR_UNSUPPORTED) return rc;
     }
-    if (g && g->exec) {
-      cudaError_t e = cudaGraphLaunch(g->exec, b->stream);
+    if (b->use_graphs && g.exec) {
+      cudaError_t e = cudaGraphLaunch(g.exec, b->stream);
       if (e != cudaSuccess) return cuda_error(e, "batch step graph");
-      b->launches += g->launches;
+      b->launches += g.launches;
     } else {
-      n = 1;
       cudaError_t e = launch_steps(b, n);
       if (e != cudaSuccess) return cuda_error(e, "batch step");
     }

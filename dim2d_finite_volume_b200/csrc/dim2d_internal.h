@@ -35,6 +35,7 @@ struct StepGraph {
   cudaGraphExec_t exec = nullptr;
   const double* A = nullptr;  // buffer that held u^n
   long long launches = 0;     // kernel launches in one replay
+  int asked = 0;              // runs that could have replayed it (batches)
 };
 // Steps per graph: a run of n steps replays as many graphs of 8 as fit, then
 // of 2 (both leave the buffer parity as it was), then of 1.  Between the
