@@ -277,18 +277,19 @@ __device__ __forceinline__ void face2(const FaceSums<T>& f, const FaceCoef<T>& c
 
 // Twice the flux of the south wall's face (wall_face_flux,
 // wall_xy_equilibrium_module.f:445-908): th = Tcl - Tcap/We of the first
-// interior node, q = wall heat flux.
+// interior node, q = wall heat flux.  In FP64 from the sums on, also in mixed
+// precision (the flux of the wall is not part of its FP32 face pass).
 template <typename T>
-__device__ __forceinline__ void wall_face2(const FaceSums<T>& f, const FaceCoef<T>& c, double th,
-                                           double dy, double q, const DimConst& k, T F[3],
-                                           double* F3) {
+__device__ __forceinline__ void wall_face2(const FaceSums<T>& f, const FaceCoef<double>& c,
+                                           double th, double dy, double q, const DimConst& k,
+                                           double F[3], double* F3) {
   const double tl = k.c38cv * th;
   const double t_half = 0.5 * (tl + (tl + dy * k.c38cv * k.re * k.pr * q));
-  const double md = 0.5 * (double)f.sr, drn = (double)(c.s * f.dr), gt = (double)f.gt;
+  const double md = 0.5 * (double)f.sr, drn = c.s * (double)f.dr, gt = (double)f.gt;
   const double p = 8.0 * md * t_half / (3.0 - md) - 3.0 * (md * md);
-  F[0] = T(0);
-  F[1] = (T)(2.0 * p - ((double)(f.sr * f.lap) + (gt * gt - drn * drn)));
-  F[2] = (T)(-2.0 * ((double)(c.b2 * f.dut) - drn * gt));
+  F[0] = 0.0;
+  F[1] = 2.0 * p - ((double)f.sr * (double)f.lap + (gt * gt - drn * drn));
+  F[2] = -2.0 * (c.b2 * (double)f.dut - drn * gt);
   *F3 = 2.0 * q;
 }
 
@@ -647,7 +648,7 @@ __device__ __forceinline__ void strip_warp(const StageArgs& a, int c0, int y0, i
   T um, vm;              // velocity of row y-1
   T ul0, vl0, gxu0, gxv0;  // row y: left velocity, undivided differences across the column
   double dn0 = r1 - r0;  // density difference between rows y and y+1
-  T Gb[3];  // in the face frame: mass, m_y, m_x
+  double Gb[3];  // in the face frame: mass, m_y, m_x
   double gb3;
   {
     const double dn = r0 - rm;
@@ -665,9 +666,13 @@ __device__ __forceinline__ void strip_warp(const StageArgs& a, int c0, int y0, i
     const FaceSums<T> s = y_sums(nm, n0, (T)dn, (T)(from_right(um) - from_left(um)), gxu0,
                                  (T)(from_right(vm) - from_left(vm)), gxv0, cd.y.th);
     if (a.wall_s && y0 == BC)
-      wall_face2(s, c.y, n0.th, a.dy, wall_heat_flux(a.wall, a.xmap0 + x * a.dx), a.k, Gb, &gb3);
-    else
-      face2(s, c.y, c.s, Gb, &gb3);
+      wall_face2(s, cd.y, n0.th, a.dy, wall_heat_flux(a.wall, a.xmap0 + x * a.dx), a.k, Gb, &gb3);
+    else {
+      T G[3];
+      face2(s, c.y, c.s, G, &gb3);
+#pragma unroll
+      for (int v = 0; v < 3; v++) Gb[v] = (double)G[v];
+    }
   }
 
   const bool active = lane >= 1 && lane <= SW && x <= f.nx - 1 - BC &&
@@ -745,9 +750,11 @@ __device__ __forceinline__ void strip_warp(const StageArgs& a, int c0, int y0, i
     // y-face between rows y and y+1
     const T ul1 = from_left(n1.u), vl1 = from_left(n1.v);
     const T gxu1 = from_right(n1.u) - ul1, gxv1 = from_right(n1.v) - vl1;
-    T Gt[3];
-    double gt3;
-    face2(y_sums(n0, n1, (T)dn0, gxu0, gxu1, gxv0, gxv1, cd.y.th), c.y, c.s, Gt, &gt3);
+    T G[3];
+    double Gt[3], gt3;
+    face2(y_sums(n0, n1, (T)dn0, gxu0, gxu1, gxv0, gxv1, cd.y.th), c.y, c.s, G, &gt3);
+#pragma unroll
+    for (int v = 0; v < 3; v++) Gt[v] = (double)G[v];
 
     // update of cell (x, y)
     const double uc[4] = {r0, mx0, my0, e0};
@@ -755,7 +762,7 @@ __device__ __forceinline__ void strip_warp(const StageArgs& a, int c0, int y0, i
 #pragma unroll
     for (int v = 0; v < 4; v++) {
       const int g = v == 1 ? 2 : (v == 2 ? 1 : 0);  // frame order of m_x and m_y
-      const double dG = v < 3 ? (double)Gb[g] - (double)Gt[g] : gb3 - gt3;
+      const double dG = v < 3 ? Gb[g] - Gt[g] : gb3 - gt3;
       q[v] = MODE != 1 ? 0.0 : need_un ? fma(a.b, un[ou + v * RC], (1.0 - a.b) * uc[v]) : uc[v];
       q[v] = fma(wx, D[v], fma(wy, dG, q[v]));
     }
