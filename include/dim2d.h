@@ -338,8 +338,9 @@ DIM2D_API int dim2d_batch_set_wait_limit(dim2d_batch *b, double seconds);
  * limit runs out; -1 (default) turns this off. */
 DIM2D_API int dim2d_batch_withhold_item(dim2d_batch *b, long long item);
 /* Autotuner: times dry steps (dt = 0, stage buffers only) of each group
- * for the 5 strip shapes and keeps the fastest; chosen[8] receives the
- * shapes, times_ms (optional) 8 x 5 dry-step times (0 for empty groups).
+ * for the 5 strip shapes and for strips by the group's size (as a new batch
+ * runs) and keeps the fastest of these six; chosen[8] receives the fastest of
+ * the 5 shapes, times_ms (optional) 8 x 5 dry-step times (0 for empty groups).
  * In persistent mode it times dry launches with 8, 16 and 32 rows per
  * strip item instead: chosen[g] receives the rows kept and times_ms[g*5 +
  * 0..2] the three times, for every g. */
