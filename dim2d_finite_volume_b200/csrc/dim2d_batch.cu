@@ -507,9 +507,7 @@ static int autotune_persistent(dim2d_batch* b, int chosen[8], double* times_ms) 
 int dim2d_batch_autotune(dim2d_batch* b, int chosen[8], double* times_ms) {
   if (!b) return set_error(DIM2D_ERR_ARG, "batch_autotune: null batch");
   if (b->persistent) return b->m.empty() ? DIM2D_OK : autotune_persistent(b, chosen, times_ms);
-  cudaEvent_t e0 = nullptr, e1 = nullptr;
-  cudaError_t e = cudaEventCreate(&e0);
-  if (e == cudaSuccess) e = cudaEventCreate(&e1);
+  cudaError_t e = cudaSuccess;
   for (int g = 0; g < NGROUPS && e == cudaSuccess; g++) {
     const std::vector<int> idx = members_of(b, g);
     double best = 1e300, best_of_five = 1e300;
@@ -530,13 +528,7 @@ int dim2d_batch_autotune(dim2d_batch* b, int chosen[8], double* times_ms) {
             r = group_stage(b, g, idx, st, sh, 0.0, b->stream);
           return r;
         };
-        e = dry();
-        if (e == cudaSuccess) e = cudaEventRecord(e0, b->stream);
-        for (int r = 0; r < 3 && e == cudaSuccess; r++) e = dry();
-        if (e == cudaSuccess) e = cudaEventRecord(e1, b->stream);
-        if (e == cudaSuccess) e = cudaEventSynchronize(e1);
-        if (e == cudaSuccess) e = cudaEventElapsedTime(&ms, e0, e1);
-        ms /= 3.0f;
+        e = time_dry_step(b->stream, b->use_graphs, dry, &b->launches, &ms);
         if (ms < best) {
           best = ms;
           best_shape = sh;
@@ -554,8 +546,6 @@ int dim2d_batch_autotune(dim2d_batch* b, int chosen[8], double* times_ms) {
     }
     if (chosen) chosen[g] = reported;
   }
-  if (e0) cudaEventDestroy(e0);
-  if (e1) cudaEventDestroy(e1);
   if (e != cudaSuccess) return cuda_error(e, "batch_autotune");
   return DIM2D_OK;
 }

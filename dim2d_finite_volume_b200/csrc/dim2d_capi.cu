@@ -521,9 +521,6 @@ int dim2d_autotune(dim2d_handle* h, int* chosen, double* times_ms) {
     }
   }
   cudaError_t e = wait_copy_if(h, h->B);  // the dry steps write B and C
-  cudaEvent_t e0, e1;
-  cudaEventCreate(&e0);
-  cudaEventCreate(&e1);
   int best = 0;
   double best_ms = 1e30;
   const int saved = h->variant;
@@ -544,24 +541,18 @@ int dim2d_autotune(dim2d_handle* h, int* chosen, double* times_ms) {
       }
       return cudaSuccess;
     };
-    e = dry_step();
-    if (e == cudaSuccess) e = cudaEventRecord(e0, h->stream);
-    const int reps = 3;
-    for (int r = 0; r < reps && e == cudaSuccess; r++) e = dry_step();
-    if (e == cudaSuccess) e = cudaEventRecord(e1, h->stream);
-    if (e == cudaSuccess) e = cudaEventSynchronize(e1);
     float ms = 0.f;
-    if (e == cudaSuccess) e = cudaEventElapsedTime(&ms, e0, e1);
+    if (e == cudaSuccess)
+      e = time_dry_step(h->stream, h->use_graphs && !h->prof && v != PERSIST_VARIANT, dry_step,
+                        &h->launches, &ms);
     if (e != cudaSuccess) break;
-    const double per = ms / reps;
+    const double per = ms;
     if (times_ms) times_ms[v] = per;
     if (per < best_ms) {
       best_ms = per;
       best = v;
     }
   }
-  cudaEventDestroy(e0);
-  cudaEventDestroy(e1);
   if (e != cudaSuccess) {
     h->variant = saved;
     return cuda_error(e, "autotune");

@@ -45,6 +45,64 @@ constexpr int GRAPH_SIZES = 3;
 constexpr int GRAPH_STEPS[GRAPH_SIZES] = {8, 2, 1};
 inline int graph_size_for(int steps) { return steps >= 8 ? 0 : steps >= 2 ? 1 : 2; }
 
+// Device time (ms) of one dry step of an autotuner, whose launches dry()
+// issues on s and counts in *launches.  With `graphs` short steps are replayed,
+// as they will be in earnest (1 ms more per field tuned): launched one by one
+// they follow at the rate of the host, 15 to 20 us per step, and every shape
+// takes as long (three periodic fields of 64^2 to 150^2 ended on a shape of
+// 22 us per step, 13 on the best; one of 128^2 even on 65, 9).
+template <typename Dry>
+cudaError_t time_dry_step(cudaStream_t s, bool graphs, Dry dry, long long* launches, float* ms) {
+  constexpr int STEPS = 2;
+  constexpr float SHORT = 0.06f;  // some three times the host's rate
+  auto steps = [&]() {
+    cudaError_t r = cudaSuccess;
+    for (int i = 0; i < STEPS && r == cudaSuccess; i++) r = dry();
+    return r;
+  };
+  cudaGraphExec_t x = nullptr;
+  long long per_replay = 0;
+  auto run = [&]() {
+    if (!x) return steps();
+    *launches += per_replay;
+    return cudaGraphLaunch(x, s);
+  };
+  cudaEvent_t e0 = nullptr, e1 = nullptr;
+  cudaError_t e = cudaEventCreate(&e0);
+  if (e == cudaSuccess) e = cudaEventCreate(&e1);
+  auto measure = [&](int reps) {
+    cudaError_t r = cudaEventRecord(e0, s);
+    for (int i = 0; i < reps && r == cudaSuccess; i++) r = run();
+    if (r == cudaSuccess) r = cudaEventRecord(e1, s);
+    if (r == cudaSuccess) r = cudaEventSynchronize(e1);
+    if (r == cudaSuccess) r = cudaEventElapsedTime(ms, e0, e1);
+    *ms /= (float)(reps * STEPS);
+    return r;
+  };
+  if (e == cudaSuccess) e = measure(1);  // warm-up
+  int reps = 1;
+  if (e == cudaSuccess && graphs && *ms < SHORT) {
+    const long long n0 = *launches;
+    if (cudaStreamBeginCapture(s, cudaStreamCaptureModeRelaxed) == cudaSuccess) {
+      e = steps();
+      cudaGraph_t g = nullptr;
+      const cudaError_t ec = cudaStreamEndCapture(s, &g);
+      if (e == cudaSuccess && ec == cudaSuccess && g) cudaGraphInstantiate(&x, g, 0);
+      if (g) cudaGraphDestroy(g);
+    }
+    cudaGetLastError();  // a stream that cannot be captured: launched
+    per_replay = *launches - n0;
+    *launches = n0;
+    if (x && e == cudaSuccess) e = run();
+    reps = 6;
+  }
+  if (e == cudaSuccess) e = measure(reps);
+  if (e0) cudaEventDestroy(e0);
+  if (e1) cudaEventDestroy(e1);
+  if (x) cudaGraphExecDestroy(x);
+  return e;
+}
+
 struct dim2d_handle {
   int device = 0;
   dim2d_params p{};
