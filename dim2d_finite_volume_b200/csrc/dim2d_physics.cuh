@@ -33,6 +33,24 @@ struct DimConst {
   double gravity;
 };
 
+// 1/d for the strip kernels' node quantities: the hardware's approximation x
+// and the first terms of the geometric series 1/d = x/(1 - e) =
+// x (1 + e + e^2 + ...), e = 1 - d x -- Chebyshev's iteration for 1/x - d
+// (J. F. Traub, Iterative Methods for the Solution of Equations, 1964).  With
+// |e| <= 2^-20 what is left out is below 2^-60, 1/128 of an ulp, so that the
+// last rounding makes the result 1.0 / d or its neighbour
+// (tests/test_reciprocal.py).  For d and 1/d normal: of zero, an infinity and
+// beyond either end of the normal range the result is NaN.  (There a node's
+// pressure is NaN with the division too: rho = 0, rho = 3 or 9 rho^2 overflowing.)
+#ifdef __CUDACC__
+__device__ __forceinline__ double reciprocal(double d) {
+  double x;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(x) : "d"(d));
+  const double e = fma(-d, x, 1.0);
+  return fma(fma(e, e, e), x, x);
+}
+#endif
+
 // Per-node primitive quantities used by the flux formulas.
 struct NodePrim {
   double u, v;   // velocity_x/y           (prim :242-289)

@@ -162,18 +162,9 @@ struct NodeQ {
 };
 
 // Primitives as node_prim() (dim2d_prim_module.f:242-289, 425-453, 515-544,
-// 1056-1071) with 1/rho and 1/(3-rho) from one division; Tcap = 0.5/rho
+// 1056-1071) with 1/rho and 1/(3-rho) from one reciprocal; Tcap = 0.5/rho
 // |grad rho|^2 with centred gradients (:582-613).  First part: what the
 // x-face of the row below takes from this row.
-// 1/d from the hardware's approximation (20 bits or better) and one step of
-// Halley's iteration, x (1 + e + e^2) with e = 1 - d x: cubic, so that the
-// remaining error is rounding (2^-60 before it).
-__device__ __forceinline__ double reciprocal(double d) {
-  double x;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(x) : "d"(d));
-  const double e = fma(-d, x, 1.0);
-  return fma(fma(e, e, e), x, x);
-}
 struct NodeUV {
   double inv, ir, u, v;
 };
