@@ -249,7 +249,6 @@ int dim2d::create_field(const dim2d_params* p, int nx, int ny, const int bc_choi
   h->precision = precision;
   h->periodic = periodic;
   h->open_all = open;
-  h->mirrors = mirrors;
   h->south_wall = south_wall;
   h->corners_y = corners_y;
   if (open) h->open_mask = OPEN_ALL;

@@ -110,7 +110,6 @@ struct dim2d_handle {
   int precision = 0;
   int periodic = 0;
   int open_all = 0;  // hedstrom_xy: every section open, type bc_timedev
-  int mirrors = 0;     // reflection_xy or wall_S_reflection (node pass kernel)
   int south_wall = 0;  // wall on S: wall_S_reflection, wall_S_open, half_wall_S_open
   int corners_y = 0;   // corner sections are reflection_y
   // open (Hedstrom) sections: dim2d::OPEN_* mask of the time-integrated ghost

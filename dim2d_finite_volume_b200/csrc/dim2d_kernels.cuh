@@ -148,8 +148,7 @@ struct StageArgs {
                                        // ghost sections; strip launches integrate those
                                        // cells too (their first CTAs)
   int mixed;                           // DIM2D_MIXED: FP32 face pass (strip kernels)
-  double t;                            // field time (constant over the stages)
-  double xmap0, ymap0;                 // x_map(1), y_map(1): x_map(i) = xmap0 + (i-1) dx
+  double xmap0;                        // x_map(1): x_map(i) = xmap0 + (i-1) dx
   int mirror;                          // NODE_* mirror sides: the strips write their ghost
                                        // images, as on a periodic field
   int wall_runs;                       // south wall: runs of wall columns whose ghost cells
@@ -215,7 +214,7 @@ struct NodeBcArgs {
   double* __restrict__ u;           // field whose ghosts are set
   Field f;
   double dx, dy, rdx, rdy;
-  double t, xmap0, ymap0;
+  double xmap0;
   int south_wall;                   // 1: wall on S, 0: mirror
   int corners_y;                    // corners are reflection_y (reflection_xy) vs _x
   int open_w, open_e, open_n;       // side open (Hedstrom, integrated by the stage):
@@ -263,9 +262,9 @@ constexpr int NUM_VARIANTS = 7;
 cudaError_t launch_time_dev(const StageArgs& a, cudaStream_t s);
 // L(u) of a buffer-layer grid at its interior_pt points (StageArgs::mask)
 cudaError_t launch_strip_masked(const StageArgs& a, cudaStream_t s);
-// open (Hedstrom) ghost cells of the sections in a.open; mode 0 writes
-// L(u) into a.uout, mode 1 the RK stage update
-cudaError_t launch_open_ghosts(const StageArgs& a, int mode, cudaStream_t s);
+// RK stage of the open (Hedstrom) ghost cells of the sections in a.open, beside
+// the tile kernel (the strips integrate them in their launch)
+cudaError_t launch_open_ghosts(const StageArgs& a, cudaStream_t s);
 cudaError_t launch_fill(double* p, double v, size_t n, cudaStream_t s);
 cudaError_t launch_periodic_ghosts(double* u, const Field& f, cudaStream_t s);
 // The ghost frame of a field: every cell within BC of an edge, 4 planes.
@@ -359,7 +358,7 @@ enum PItemType : int { PI_GHOST = 0, PI_STRIP = 1, PI_NODE = 2 };
 struct PDomain {
   Field f;
   double* buf[3];  // at launch: [0] = u^n, [1] = the other buffer of the pair, [2] = C
-  double dx, dy, rdx, rdy, dt, xmap0, ymap0;
+  double dx, dy, rdx, rdy, dt, xmap0;
   int periodic, wall_s, open;                        // as StageArgs
   int south_wall, corners_y, open_w, open_e, open_n;  // as NodeBcArgs
   int sx;                                            // strips per row band

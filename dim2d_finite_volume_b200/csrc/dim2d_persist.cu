@@ -154,7 +154,6 @@ int persist_build(PersistPlan& pl, const std::vector<dim2d_handle*>& hs,
     d.rdy = h->rdy;
     d.dt = dts[j];
     d.xmap0 = h->xmap0;
-    d.ymap0 = h->ymap0;
     d.periodic = h->periodic;
     d.wall_s = h->south_wall;
     d.open = h->open_mask;

@@ -31,9 +31,7 @@ StageArgs make_stage_args(const dim2d_handle* h, const double* uin, double* uout
   a.variant = h->variant;
   a.open = h->open_mask;
   a.mixed = h->precision == DIM2D_MIXED;
-  a.t = h->t;
   a.xmap0 = h->xmap0;
-  a.ymap0 = h->ymap0;
   // every other launch of a run of steps (A and B change places each step)
   a.reverse = (st & 1) ^ (h->A < h->B);
   a.mirror = h->mirror_sides;
@@ -56,9 +54,7 @@ static NodeBcArgs make_node_args(const dim2d_handle* h, const double* utmp, doub
   a.dy = h->dy;
   a.rdx = h->rdx;
   a.rdy = h->rdy;
-  a.t = h->t;
   a.xmap0 = h->xmap0;
-  a.ymap0 = h->ymap0;
   a.south_wall = h->south_wall;
   a.corners_y = h->corners_y;
   a.open_w = h->open_w;
@@ -143,7 +139,7 @@ cudaError_t launch_stage_work(dim2d_handle* h, const StageArgs& a, int mode) {
     e = launch_open_runs(corners, mode, h->stream);
     h->launches++;
   } else if (!stage_fuses_open(a)) {
-    e = launch_open_ghosts(a, mode, h->stream);
+    e = launch_open_ghosts(a, h->stream);
     h->launches++;
   }
   return e;

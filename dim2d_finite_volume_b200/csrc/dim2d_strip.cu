@@ -244,7 +244,7 @@ struct FaceSums {
 };
 
 // Twice the face flux of (mass, normal momentum, tangential momentum,
-// energy); formulas of face_flux_t (dim2d_fluxes_module.f:103-541) on sums
+// energy); formulas of face_flux (dim2d_fluxes_module.f:103-541) on sums
 // instead of averages.  tnn, tnt: viscous stress plus the capillary terms
 // that enter the energy flux with the same velocity.
 // The temperature term of the energy flux, which holds the third
@@ -1014,9 +1014,7 @@ __device__ __forceinline__ StageArgs batch_stage_args(const BatchStageArgs& P, i
   a.wc = d.wc;
   a.reverse = 0;
   a.mixed = 0;
-  a.t = 0.0;
   a.xmap0 = d.xmap0;
-  a.ymap0 = 0.0;
   a.wall = P.wall;
   a.k = P.k;
   a.c = d.c;
@@ -1156,9 +1154,7 @@ __device__ __forceinline__ NodeBcArgs persist_node_args(const PersistArgs& P, co
   a.dy = d.dy;
   a.rdx = d.rdx;
   a.rdy = d.rdy;
-  a.t = 0.0;
   a.xmap0 = d.xmap0;
-  a.ymap0 = d.ymap0;
   a.south_wall = d.south_wall;
   a.corners_y = d.corners_y;
   a.open_w = d.open_w;
