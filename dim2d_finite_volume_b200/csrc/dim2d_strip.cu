@@ -941,7 +941,7 @@ enum StripEdges : int { E_NONE = 0, E_OPEN = 1, E_WALL = 2 };
 
 // CTA number b of one field (one warp per CTA): its edge_ctas edge runs, then
 // its strips, sx per band of h rows, x fastest.
-template <int MODE, int UN, int EDGES, bool MIX>
+template <int MODE, int UN, int EDGES, bool MIX, bool BATCH = false>
 __device__ __forceinline__ void strip_cta(const StageArgs& a, int b, int edge_ctas, int sx, int h) {
   constexpr bool WALLS = MODE == 1 && EDGES == E_WALL;
   bool wall = false;
@@ -960,9 +960,11 @@ __device__ __forceinline__ void strip_cta(const StageArgs& a, int b, int edge_ct
   int y0 = (MODE >= 2 ? a.box_y0 : BC) + (b / sx) * h;
   const int ylast = MODE >= 2 ? a.box_y1 : a.f.ny - BC - 1;
   int y1 = min(y0 + h, ylast + 1);
-  // (Every strip has a row and a column.  The tests make a warp compute its place
-  // before it waits for the launch before; without them that moves behind the
-  // wait: 128^2 periodic 8.97 us per step, 8.46 so, 512^2 wall 25.58, 25.36.)
+  // Every strip has a row and a column.  The test makes a warp compute its place
+  // before it waits for the launch before; without it that moves behind the wait:
+  // 128^2 periodic 8.97 us per step, 8.46 so, 512^2 wall 25.58, 25.36.  (Not in
+  // batches, which look their domain up before and have no registers for it.)
+  auto some = [&]() { return BATCH || (c0 < a.f.nx && y0 < y1); };
   if (WALLS) {
     const WallRun run(a, b);
     if (wall) {
@@ -970,10 +972,10 @@ __device__ __forceinline__ void strip_cta(const StageArgs& a, int b, int edge_ct
       y0 = BC;
       y1 = BC + 2;
     }
-    if (c0 < a.f.nx && y0 < y1) strip_warp<MODE, UN, MIX, true>(a, c0, y0, y1, wall);
+    if (some()) strip_warp<MODE, UN, MIX, true>(a, c0, y0, y1, wall);
     if (wall) wall_columns(a, run);
   } else {
-    if (c0 < a.f.nx && y0 < y1) strip_warp<MODE, UN, MIX>(a, c0, y0, y1);
+    if (some()) strip_warp<MODE, UN, MIX>(a, c0, y0, y1);
   }
 }
 
@@ -1051,8 +1053,8 @@ __global__ void __launch_bounds__(32, WARPS)
   const StageArgs a = batch_stage_args<MIX>(P, i);
   const BatchDomain& d = P.d[i];
   // its edge runs are numbered from 0, its strips from edge_ctas
-  strip_cta<1, UN, EDGES, MIX>(a, edge ? b - d.edge0 : P.edge_ctas + b - d.strip0, P.edge_ctas,
-                               d.sx, h);
+  strip_cta<1, UN, EDGES, MIX, true>(a, edge ? b - d.edge0 : P.edge_ctas + b - d.strip0,
+                                     P.edge_ctas, d.sx, h);
 }
 
 // ---- persistent batched kernel -----------------------------------------
