@@ -126,7 +126,7 @@ struct dim2d_handle {
   unsigned int* status = nullptr;  // wall root status word (device)
   double xmap0 = 0, ymap0 = 0;     // x_map(1), y_map(1)
   int variant = 0;                 // stage-kernel variant (dim2d_set_variant)
-  bool uncounted = false;          // step_noalloc: no caller counts its launches
+  bool corners_apart = true;       // variant 0, hedstrom_xy: see launch_stage_work
   struct dim2d_batch* batch = nullptr;  // batch this field belongs to, if any
   // dim2d_download_async: side stream, its events, and the buffer being copied
   cudaStream_t copy_stream = nullptr;

@@ -168,7 +168,7 @@ extern "C" int dim2d_step_noalloc(const dim2d_params* p, int nx, int ny, const i
   h.p = *p;
   h.k = make_const(*p);
   h.precision = DIM2D_FP64;
-  h.uncounted = true;
+  h.corners_apart = false;
   h.periodic = periodic;
   h.open_all = open;
   h.open_mask = open ? OPEN_ALL : 0;

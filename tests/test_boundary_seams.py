@@ -175,6 +175,29 @@ def test_graphs_of_eight_steps_bit_identical(oracle, wall, preset, variant):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("n, ny", [(8, 8), (61, 33), (130, 64)])
+@pytest.mark.parametrize("graphs", [True, False])
+def test_corner_cells_in_the_launch_of_a_long_run(oracle, n, ny, graphs):
+    """An untuned open field: one kernel per stage in runs of eight steps, two in
+    the steps that remain and in shorter runs, with the same bits."""
+    from dim2d_finite_volume_b200 import field as F
+    _, d, _ = _case(oracle, "hedstrom_xy", n, ny)
+    got = []
+    for runs, kernels in (((16, 3), 16 * 3 + 3 * 6), ((4, 4, 4, 4, 3), 19 * 6)):
+        with F.Field(d["nx"], d["ny"], bc="hedstrom_xy", params=F.default_params()) as f:
+            f.set_graphs(graphs)
+            f.ini(d["nodes"], d["x_map"], d["y_map"])
+            n0 = f.launches
+            for steps in runs:
+                f.integrate(0.5 * d["dt"], steps)
+            assert f.launches - n0 == kernels
+            got.append((f.download(), f.compute_time_dev()))
+    assert np.isfinite(got[0][0]).all()
+    for v in range(2):
+        assert np.array_equal(got[0][v], got[1][v])
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("preset", ["periodic_xy", "hedstrom_xy", "wall_S_open"])
 def test_asynchronous_copy_before_a_long_run(oracle, wall, preset):
     """A copy of the state queued before runs of eight steps and more holds that
