@@ -22,8 +22,8 @@
 // One thread per ghost cell; the state is read straight from global memory
 // (the ghost ring is a few rows, L2-resident), the output is written with
 // the same RK3 stage update as the interior kernel.  Included by
-// dim2d_open.cu (stand-alone ghost kernel) and dim2d_strip.cu (ghost
-// cells fused into the stage launch as its first CTAs).
+// dim2d_open.cu, the ghost kernel beside the tile kernel; stage launches of
+// strips integrate these cells by runs (open_run, dim2d_strip.cu).
 #pragma once
 #include "dim2d_kernels.cuh"
 

@@ -30,8 +30,9 @@
 // 165 128-byte wavefronts per warp and row through that pipe, against 121
 // cycles of FP64 work; now a row costs 34 shuffles, 36 wavefronts of row data
 // and 165 FP64 instructions instead of 242.  Measured per RK3 step (best
-// shape): 1024^2 periodic 99.7 -> 70.2 us, 2048^2 open 321.7 -> 226.8 us,
-// 2048^2 wall in mixed precision 324.8 -> 223.0 us.  Tried beside it: all
+// shape): 1024^2 periodic 99.7 -> 70.1 us, 2048^2 open 321.7 -> 230, 2048^2 wall
+// in mixed precision 324.8 -> 223 in runs of some 10 ms; longer ones at 2048^2
+// reach the board's power limit (open 257 to 270).  Tried beside it: all
 // rows prefetched into registers instead of the ring (periodic 85.7, more
 // registers and 420 instead of 400 instructions per row), 20 warps per SM at
 // 96 registers (92; spills), three or four rows per pass (as fast, larger).
@@ -1280,13 +1281,13 @@ constexpr int SHAPE_ROWS[5] = {8, 16, 32, 4, 2};
 // one strip; 16 where even those do not fit (more rows leave the last wave
 // emptier, fewer repeat the two rows below a strip more often).  us per step:
 //   rows                       by size    2      4      8      16
-//   64^2 open                   9.2 (1)    8.9   10.5   14.9   24.3
-//   128^2 periodic              8.5 (1)   10.5   14.1   21.5   36.1
-//   301x187 half_wall_S_open   21.9 (2)   20.9   20.4   22.3   37.4
-//   512^2 wall_S_reflection    25.2 (4)   30.0   25.2   26.9   38.5
-//   1024^2 open                69.1 (16)  88.1   73.6   68.0   66.3
-//   1531x1117 periodic         110 (16)   141    116    107    110
-//   2048^2 open                227 (16)   328    264    236    230
+//   64^2 open                   8.5 (1)    8.3   10.1   14.9   24.3
+//   128^2 periodic              8.5 (1)   10.0   13.6   21.2   36.3
+//   301x187 half_wall_S_open   21.8 (2)   20.7   20.4   22.2   36.6
+//   512^2 wall_S_reflection    25.1 (4)   29.8   25.1   27.1   38.8
+//   1024^2 open                66.2 (16)  88.4   73.9   68.2   67.2
+//   1531x1117 periodic         109 (16)   140    115    108    110
+//   2048^2 open                230 (16)   335    272    251    232
 template <typename Strips>
 int rows_of(int shape, Strips strips) {
   if (shape != SHAPE_BY_SIZE) return SHAPE_ROWS[shape];

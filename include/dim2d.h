@@ -84,10 +84,10 @@ extern "C" {
 
 /* precision of the stencil/flux pass.  DIM2D_MIXED: the node pass (van der
  * Waals inversion for velocities, pressure, temperatures) runs in FP64 and
- * leaves FP32 copies of the node state and quantities in shared memory; the
- * face pass (stencils and flux formulas) reads those FP32 copies and runs in
- * FP32, except the third-derivative capillary term (normal derivative of
- * the capillary temperature), which stays FP64; divergence and RK
+ * rounds the node state and quantities to FP32; the face pass (sums,
+ * differences and flux formulas) runs on those in FP32, except the
+ * temperature term of the energy flux (with the third derivatives of its
+ * capillary part) and the flux of a wall, which stay FP64; divergence and RK
  * accumulation are FP64 on the FP64 state in HBM.  Error against the FP64
  * path: <= 1e-5 normwise on the state (see the library's tests). */
 #define DIM2D_FP64 0
