@@ -352,8 +352,13 @@ __host__ __device__ inline void node_bc_cell(const NodeBcArgs& a, int m) {
     in.gmx = ld(a.utmp, f, 1, x, 2);
     in.gmy = ld(a.utmp, f, 2, x, 2);
     in.gE = ld(a.utmp, f, 3, x, 2);
-    if (gt != WG_L0) in.grw = ld(a.utmp, f, 0, x - 1, 2);
-    if (gt != WG_R0) in.gre = ld(a.utmp, f, 0, x + 1, 2);
+    // (in place, a mirror side's ghost cells are being written by this launch:
+    // read at their source)
+    const bool in_place = a.utmp == u;
+    const int xw = in_place && x - 1 < BC && !a.open_w ? mirror_lo_hi(x - 1, nx) : x - 1;
+    const int xe = in_place && x + 1 >= nx - BC && !a.open_e ? mirror_lo_hi(x + 1, nx) : x + 1;
+    if (gt != WG_L0) in.grw = ld(a.utmp, f, 0, xw, 2);
+    if (gt != WG_R0) in.gre = ld(a.utmp, f, 0, xe, 2);
     in.grs = ld(a.utmp, f, 0, x, 1);
     in.grn = ld(a.utmp, f, 0, x, 3);
     in.r1 = ld(u, f, 0, x, 2);
