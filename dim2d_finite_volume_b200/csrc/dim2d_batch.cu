@@ -517,7 +517,11 @@ int dim2d_batch_autotune(dim2d_batch* b, int chosen[8], double* times_ms) {
     // strips by size too: few small fields run fastest on strips of one row,
     // which no shape has (one 128^2 periodic field: 8.5 us per step, 10.5 on
     // strips of two rows)
-    for (int sh = SHAPE_BY_SIZE; sh < NSHAPES && e == cudaSuccess; sh++) {
+    // (timed first and once more at the end: the first finds the device idle)
+    constexpr int ORDER[] = {SHAPE_BY_SIZE, 0, 1, 2, 3, 4, SHAPE_BY_SIZE};
+    static_assert(NSHAPES == 5, "shapes of ORDER");
+    for (int sh : ORDER) {
+      if (e != cudaSuccess) break;
       float ms = 0.f;
       if (!idx.empty()) {
         // dry steps (dt = 0) of this group alone: the stages write the

@@ -523,7 +523,9 @@ int dim2d_autotune(dim2d_handle* h, int* chosen, double* times_ms) {
   int best = 0;
   double best_ms = 1e30;
   const int saved = h->variant;
-  for (int v = 0; v < NUM_VARIANTS; v++) {
+  // variant 0 first and once more at the end: the first finds the device idle
+  for (int i = 0; i <= NUM_VARIANTS; i++) {
+    const int v = i % NUM_VARIANTS;
     h->variant = v;
     // a dry RK3 step: the three stages with their boundary passes, dt = 0,
     // writing only the stage buffers B and C (A, the state, is read only
@@ -546,7 +548,7 @@ int dim2d_autotune(dim2d_handle* h, int* chosen, double* times_ms) {
                         &h->launches, &ms);
     if (e != cudaSuccess) break;
     const double per = ms;
-    if (times_ms) times_ms[v] = per;
+    if (times_ms) times_ms[v] = i < NUM_VARIANTS ? per : std::min(times_ms[v], per);
     if (per < best_ms) {
       best_ms = per;
       best = v;

@@ -2,6 +2,8 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <algorithm>
+#include <chrono>
 #include <cstdarg>
 #include <vector>
 
@@ -46,15 +48,15 @@ constexpr int GRAPH_STEPS[GRAPH_SIZES] = {8, 2, 1};
 inline int graph_size_for(int steps) { return steps >= 8 ? 0 : steps >= 2 ? 1 : 2; }
 
 // Device time (ms) of one dry step of an autotuner, whose launches dry()
-// issues on s and counts in *launches.  With `graphs` short steps are replayed,
-// as they will be in earnest (1 ms more per field tuned): launched one by one
-// they follow at the rate of the host, 15 to 20 us per step, and every shape
-// takes as long (three periodic fields of 64^2 to 150^2 ended on a shape of
-// 22 us per step, 13 on the best; one of 128^2 even on 65, 9).
+// issues on s and counts in *launches.  Where issuing a step takes the host more
+// than half of the step's time, steps are replayed with `graphs`, as they will be
+// in earnest: launched one by one they follow at the rate of the host, 15 us per
+// step of a field, 60 us of a batch, and every shape takes as long (three periodic
+// fields of 64^2 to 150^2 ended on a shape of 22 us per step, 13 on the best; one
+// of 128^2 even on 65, 9).
 template <typename Dry>
 cudaError_t time_dry_step(cudaStream_t s, bool graphs, Dry dry, long long* launches, float* ms) {
   constexpr int STEPS = 2;
-  constexpr float SHORT = 0.06f;  // some three times the host's rate
   auto steps = [&]() {
     cudaError_t r = cudaSuccess;
     for (int i = 0; i < STEPS && r == cudaSuccess; i++) r = dry();
@@ -70,9 +72,13 @@ cudaError_t time_dry_step(cudaStream_t s, bool graphs, Dry dry, long long* launc
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   cudaError_t e = cudaEventCreate(&e0);
   if (e == cudaSuccess) e = cudaEventCreate(&e1);
+  float issue = 0.f;
   auto measure = [&](int reps) {
     cudaError_t r = cudaEventRecord(e0, s);
+    const auto t0 = std::chrono::steady_clock::now();
     for (int i = 0; i < reps && r == cudaSuccess; i++) r = run();
+    const std::chrono::duration<float, std::milli> t = std::chrono::steady_clock::now() - t0;
+    issue = t.count() / (float)(reps * STEPS);
     if (r == cudaSuccess) r = cudaEventRecord(e1, s);
     if (r == cudaSuccess) r = cudaEventSynchronize(e1);
     if (r == cudaSuccess) r = cudaEventElapsedTime(ms, e0, e1);
@@ -80,8 +86,8 @@ cudaError_t time_dry_step(cudaStream_t s, bool graphs, Dry dry, long long* launc
     return r;
   };
   if (e == cudaSuccess) e = measure(1);  // warm-up
-  int reps = 1;
-  if (e == cudaSuccess && graphs && *ms < SHORT) {
+  if (e == cudaSuccess) e = measure(1);
+  if (e == cudaSuccess && graphs && issue > 0.5f * *ms) {
     const long long n0 = *launches;
     if (cudaStreamBeginCapture(s, cudaStreamCaptureModeRelaxed) == cudaSuccess) {
       e = steps();
@@ -93,10 +99,17 @@ cudaError_t time_dry_step(cudaStream_t s, bool graphs, Dry dry, long long* launc
     cudaGetLastError();  // a stream that cannot be captured: launched
     per_replay = *launches - n0;
     *launches = n0;
+    // the least of four, some 0.15 ms each after the first
     if (x && e == cudaSuccess) e = run();
-    reps = 6;
+    float least = *ms;
+    int reps = 1;
+    for (int r = 0; r < 4 && x && e == cudaSuccess; r++) {
+      e = measure(reps);
+      least = std::min(least, *ms);
+      reps = std::max(1, std::min(6, (int)(0.15f / (least * STEPS))));
+    }
+    *ms = least;
   }
-  if (e == cudaSuccess) e = measure(reps);
   if (e0) cudaEventDestroy(e0);
   if (e1) cudaEventDestroy(e1);
   if (x) cudaGraphExecDestroy(x);
